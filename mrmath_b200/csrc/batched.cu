@@ -608,7 +608,7 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
     const size_t bytes_i = (size_t)count * 4, bytes_l = (size_t)count * 8;
     const size_t plan_bytes = 3 * bytes_i + 2 * bytes_l + 256;
     void* pplan;
-    B2M_TRY(ws_get(ctx, kWsH, plan_bytes + 256, &pplan));
+    B2M_TRY(ws_get(ctx, kWsPlan, plan_bytes + 256, &pplan));
     char* pp = static_cast<char*>(pplan);
     int32_t* dn = reinterpret_cast<int32_t*>(pp);
     int32_t* dk = dn + count;

@@ -46,6 +46,8 @@ enum WsSlot : int {
     kWsH,
     kWsPmap,       // row maps of the blocked FP64 LU's outer panels
     kWsTri,        // the FP64 blocked sweeps' diagonal inverses, coupling blocks and published blocks
+    kWsPlan,       // the batched solve's plan: read again by later calls with the same plan, so no other
+                   // routine may write here
     kNumWs
 };
 
