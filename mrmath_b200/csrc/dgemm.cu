@@ -46,6 +46,7 @@ struct DgemmArgs {
     int op;
     int32_t* status;
     int check_info;
+    int lower;  // only tiles that reach C's lower triangle (row >= column) are computed
 };
 
 __device__ __forceinline__ void dmma16x8x4(double (&d)[4], double a0, double a1, double b0) {
@@ -81,6 +82,8 @@ __global__ void __launch_bounds__(T::kThreads, T::kCtas)
     const int in_group = bid % (kGroupM * tiles_n);
     const int tm = first_m + in_group % gsize;
     const int tn = in_group / gsize;
+
+    if (p.lower && tn * BN >= (tm + 1) * BM) return;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int KT = (p.K + BKD - 1) / BKD;
@@ -320,7 +323,7 @@ __global__ void dgemm_ktail_kernel(const double* A, int64_t lda, int64_t ar0, in
 }  // namespace
 
 int32_t dgemm_tiled(Ctx* ctx, cudaStream_t st, const DOperand& A, const DOperand& B, double* C, int64_t ldc, int64_t M,
-                    int64_t N, int64_t K, int op, bool check_info) {
+                    int64_t N, int64_t K, int op, bool check_info, bool lower) {
     if (M <= 0 || N <= 0) return B2M_OK;
     if (K <= 0) {
         if (op == B2M_DO_NONE) B2M_CU(ctx, cudaMemset2DAsync(C, ldc * 8, 0, N * 8, M, st));
@@ -335,7 +338,7 @@ int32_t dgemm_tiled(Ctx* ctx, cudaStream_t st, const DOperand& A, const DOperand
         const int64_t K16 = K & ~int64_t(15);
         int tail_op = op;
         if (K16 > 0) {
-            B2M_TRY(dgemm_tiled(ctx, st, A, B, C, ldc, M, N, K16, op, check_info));
+            B2M_TRY(dgemm_tiled(ctx, st, A, B, C, ldc, M, N, K16, op, check_info, lower));
             if (op == B2M_DO_NONE) tail_op = B2M_DO_ADD;
         }
         const int64_t outs = M * N;
@@ -358,6 +361,7 @@ int32_t dgemm_tiled(Ctx* ctx, cudaStream_t st, const DOperand& A, const DOperand
     a.C = C; a.ldc = ldc; a.op = op;
     a.status = ctx->d_status;
     a.check_info = check_info ? 1 : 0;
+    a.lower = lower ? 1 : 0;
     switch (pick_tile(ctx, M, N, K)) {
         case 128: return launch_tile<DgTile128>(ctx, st, A, B, a);
         case 64: return launch_tile<DgTile64>(ctx, st, A, B, a);

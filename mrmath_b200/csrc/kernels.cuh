@@ -18,9 +18,15 @@ struct DOperand {
 
 // C(M x N) op= A(M x K) * B(K x N) in FP64 on the DMMA path.  Tensor-map origins c0 must be
 // even; any K works (a k range that ends inside the maps off the 16-wide k-tile runs its last
-// K % 16 columns as a separate short-K pass).
+// K % 16 columns as a separate short-K pass).  lower: only the elements on and below C's diagonal are
+// wanted (tiles strictly above it are skipped; other elements above it may or may not be written).
 int32_t dgemm_tiled(Ctx* ctx, cudaStream_t st, const DOperand& A, const DOperand& B, double* C, int64_t ldc,
-                    int64_t M, int64_t N, int64_t K, int op, bool check_info);
+                    int64_t M, int64_t N, int64_t K, int op, bool check_info, bool lower = false);
+
+// A[r][c] -= sum_k L[r][c0 + k] L[c][c0 + k] for columns c in [cl, ch) and rows r >= c (tiles that
+// reach the lower triangle), k < 32: a Cholesky leaf's update of the rest of its outer panel (lu.cu).
+int32_t chol_panel_update(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t n, int64_t c0, int64_t cl,
+                          int64_t ch);
 
 // Partial-pivoting LU of the leading n x n block of a row-major FP64 array (ld even, base
 // 16-byte aligned), in place.  ipiv (device, n int32) gets absolute pivot rows; perm (device,

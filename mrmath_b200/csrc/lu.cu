@@ -270,7 +270,9 @@ __global__ void __launch_bounds__(kSuThreads)
 // leaf's rank-w update of the rest of its outer panel.  64 x 64 tiles, 4 x 4 per thread, the
 // L21 and U12 slices staged in shared memory; the w products of each element are accumulated in
 // ascending k and subtracted once (as the GEMM's doSub epilogue does).
+// kSym (a Cholesky leaf): U12 is L21^T, and tiles strictly above the diagonal are left out.
 constexpr int kRuT = 64;
+template <bool kSym>
 __global__ void __launch_bounds__(256, 2) panel_rank_update_kernel(double* A, int64_t ld, int n, int r_lo, int cl, int ch,
                                                           int c0, int w, const int32_t* status) {
     __shared__ double s_a[kRuT][kPanelW + 1];  // L21 rows of the tile
@@ -280,6 +282,7 @@ __global__ void __launch_bounds__(256, 2) panel_rank_update_kernel(double* A, in
     const int tiles_x = (ch - cl + kRuT - 1) / kRuT, tiles = tiles_x * ((n - r_lo + kRuT - 1) / kRuT);
     for (int tl = blockIdx.x; tl < tiles; tl += gridDim.x) {  // a grid smaller than the tiles loops
         const int r0 = r_lo + (tl / tiles_x) * kRuT, cb = cl + (tl % tiles_x) * kRuT;
+        if (kSym && r0 + kRuT <= cb) continue;
         batched_copy<256, kRuT * kPanelW / 256, double>(t, kRuT * kPanelW,
             [&](int e) {
                 const int rr = e >> 5, k = e & 31, row = r0 + rr;
@@ -288,10 +291,11 @@ __global__ void __launch_bounds__(256, 2) panel_rank_update_kernel(double* A, in
             [&](int e, double v) { s_a[e >> 5][e & 31] = v; });
         batched_copy<256, kPanelW * kRuT / 256, double>(t, kPanelW * kRuT,
             [&](int e) {
-                const int k = e / kRuT, col = cb + e % kRuT;
-                return (k < w && col < ch) ? A[(int64_t)(c0 + k) * ld + col] : 0.0;
+                const int k = kSym ? e & 31 : e / kRuT, col = cb + (kSym ? e >> 5 : e % kRuT);
+                if (k >= w || col >= ch) return 0.0;
+                return kSym ? A[(int64_t)col * ld + c0 + k] : A[(int64_t)(c0 + k) * ld + col];
             },
-            [&](int e, double v) { s_b[e / kRuT][e % kRuT] = v; });
+            [&](int e, double v) { s_b[kSym ? e & 31 : e / kRuT][kSym ? e >> 5 : e % kRuT] = v; });
         // the tile's own values, loaded while the slices arrive
         double c[4][4];
     #pragma unroll
@@ -791,7 +795,7 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
             if (ch <= cl || rl >= n) return B2M_OK;
             const int64_t tiles = ceil_div(ch - cl, kRuT) * ceil_div(n - rl, kRuT);
             prof_begin(ctx, qs, kClsGemm);
-            B2M_CU(ctx, launch_k(ctx, panel_rank_update_kernel, dim3((unsigned)std::min<int64_t>(tiles, max_ctas)),
+            B2M_CU(ctx, launch_k(ctx, panel_rank_update_kernel<false>, dim3((unsigned)std::min<int64_t>(tiles, max_ctas)),
                                  dim3(256), 0, qs, A, ld, (int)n, (int)rl, (int)cl, (int)ch, (int)c0, (int)wl,
                                  (const int32_t*)ctx->d_status));
             prof_end(ctx, qs, kClsGemm, 2.0 * (double)(n - rl) * (double)(ch - cl) * (double)wl);  // flops
@@ -887,6 +891,18 @@ int32_t ensure_side_stream(Ctx* ctx) {
     B2M_CU(ctx, cudaEventCreateWithFlags(&ctx->ev_leaf_panel, cudaEventDisableTiming));
     B2M_CU(ctx, cudaEventCreateWithFlags(&ctx->ev_leaf_side, cudaEventDisableTiming));
     ctx->chain_priority = greatest;
+    return B2M_OK;
+}
+
+int32_t chol_panel_update(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t n, int64_t c0, int64_t cl,
+                          int64_t ch) {
+    if (ch <= cl) return B2M_OK;
+    const int64_t tiles = ceil_div(ch - cl, kRuT) * ceil_div(n - cl, kRuT);
+    prof_begin(ctx, st, kClsGemm);
+    B2M_CU(ctx, launch_k(ctx, panel_rank_update_kernel<true>, dim3((unsigned)tiles), dim3(256), 0, st, A, ld, (int)n,
+                         (int)cl, (int)cl, (int)ch, (int)c0, kPanelW, (const int32_t*)ctx->d_status));
+    prof_end(ctx, st, kClsGemm, 2.0 * (double)(n - cl) * (double)(ch - cl) * kPanelW);  // flops
+    B2M_LAUNCHED(ctx);
     return B2M_OK;
 }
 
