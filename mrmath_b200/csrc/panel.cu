@@ -487,7 +487,7 @@ __global__ void __launch_bounds__(kPNa, 1)
     __shared__ __align__(16) uint32_t s_key[2][kPNw];       // leading words of s_loc's values
     __shared__ __align__(16) double s_u[kPW][kPW];              // rows of U
     __shared__ __align__(16) double s_l[kPBk][kPBk];        // the block's rows of L11
-    __shared__ __align__(8) uint64_t s_bar[2], s_rbar;
+    __shared__ __align__(8) uint64_t s_bar[kPSlots], s_rbar;    // a column's candidates; a block's pivot rows
     __shared__ int s_pl[kPW], s_ps[kPW];                        // the pivots: local row, CTA
     if (status[kInfo] != 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -495,13 +495,15 @@ __global__ void __launch_bounds__(kPNa, 1)
     const int nr = max(0, min(m, lo + R) - lo);
     if constexpr (MULTI) {
         // every CTA's barriers are initialised before the first push; the wait comes after the loads
+        // One barrier per candidate slot: the scribe may be up to a block of columns behind the main
+        // warps, and must not miss a phase (with two barriers, two columns on, it would wait for one
+        // that has passed).
         if (tid == 0) {
-            mbar_init(&s_bar[0], 1);
-            mbar_init(&s_bar[1], 1);
+            for (int j = 0; j < kPSlots; ++j) mbar_init(&s_bar[j], 1);
             mbar_init(&s_rbar, 1);
             fence_barrier_init();
-            mbar_arrive_expect_tx(&s_bar[0], (uint32_t)(C * kPNw * 16 * cand_pieces(0)));
-            if (w > 1) mbar_arrive_expect_tx(&s_bar[1], (uint32_t)(C * kPNw * 16 * cand_pieces(1)));
+            for (int j = 0; j < min(kPSlots, w); ++j)
+                mbar_arrive_expect_tx(&s_bar[j], (uint32_t)(C * kPNw * 16 * cand_pieces(j)));
             mbar_arrive_expect_tx(&s_rbar, (uint32_t)(min(kPBk, w) * kPW * 8));
         }
         __syncwarp();
@@ -587,7 +589,7 @@ __global__ void __launch_bounds__(kPNa, 1)
         if (!late) atomicExch(&status[kTimeout], site);
         late = true;
     };
-    auto wait_col = [&](const int j) { wait_bar(&s_bar[j & 1], (j >> 1) & 1, 201); };
+    auto wait_col = [&](const int j) { wait_bar(&s_bar[j & (kPSlots - 1)], j / kPSlots, 201); };
     bool stop = false;
     if (warp == kPNw) {
         // ---- scribe warp: records each pivot, and the pivot row's part of U inside its block
@@ -703,7 +705,7 @@ __global__ void __launch_bounds__(kPNa, 1)
                 const uint4* src = reinterpret_cast<const uint4*>(&s_loc[slot][warp]);
                 const int np = cand_pieces(col);
                 const uint32_t rdst = push_dst + slot * (uint32_t)(kPNw * kPMaxC * sizeof(PCand));
-                const uint32_t rbar = push_bar + 8 * (col & 1);
+                const uint32_t rbar = push_bar + 8 * slot;
                 if ((lane & 15) < C)
                     for (int q = lane >> 4; q < np; q += 2) st_async16(rdst + 16 * q, src[q], rbar);
             }
@@ -716,8 +718,9 @@ __global__ void __launch_bounds__(kPNa, 1)
                 const int j = jb + t;
                 if constexpr (MULTI) {
                     wait_col(j);
-                    if (tid == 0 && j + 2 < w)
-                        mbar_arrive_expect_tx(&s_bar[j & 1], (uint32_t)(C * kPNw * 16 * cand_pieces(j + 2)));
+                    if (tid == 0 && j + kPSlots < w)
+                        mbar_arrive_expect_tx(&s_bar[j & (kPSlots - 1)],
+                                              (uint32_t)(C * kPNw * 16 * cand_pieces(j + kPSlots)));
                 } else {
                     asm volatile("bar.sync 1, %0;\n" ::"r"(kPNa) : "memory");
                 }
