@@ -252,10 +252,6 @@ __device__ __forceinline__ unsigned long long ds_ld64(const unsigned long long* 
 __device__ __forceinline__ void ds_st64(unsigned long long* p, unsigned long long v) {
     asm volatile("st.relaxed.gpu.global.b64 [%0], %1;\n" ::"l"(p), "l"(v) : "memory");
 }
-__device__ __forceinline__ void cp_async8(void* dst, const void* src, int src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes)
-                 : "memory");
-}
 
 // T_bj (64 x 64) into shared memory as 64 lines of kDsTS doubles: line r holds row r of T_bj for the
 // row-major triangles (L, U), line c holds column c for the transposed ones (U^T, L^T) -- in both

@@ -111,9 +111,17 @@ int32_t lu_determinant(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld, 
 
 // Factors one m x w panel (w <= 32, row stride ld) with partial pivoting on one thread-block
 // cluster; ipiv[col_base + j] = row_base + pivot row.  panel_max_rows: tallest panel supported.
+// link (up to 8192 rows): moves_out receives the leaf's interchanges as moves; moves_in not null: the
+// 32 columns left of the panel are the leaf before it, whose interchanges (these moves), triangular
+// solve and update the panel's columns still lack, its top rows 32 rows above P included.
+constexpr int kPanelMoves = 128;  // ints of one moves buffer
+struct PanelLink {
+    const int32_t* moves_in = nullptr;
+    int32_t* moves_out = nullptr;
+};
 template <typename T>
 int32_t launch_panel(Ctx* ctx, cudaStream_t st, T* P, int64_t ld, int m, int w, int row_base, int col_base,
-                     int32_t* ipiv);
+                     int32_t* ipiv, const PanelLink& link = PanelLink());
 int panel_max_rows(bool fp64, int w);
 
 // Copies a strided FP64 matrix (rows x cols, byte strides) device to device.

@@ -266,6 +266,96 @@ __global__ void __launch_bounds__(kSuThreads)
     }
 }
 
+// A linked leaf [c0, c0 + w) (panel_kernel): its interchanges, given as moves, on the outer panel's
+// columns left of it, [k0, c0), and on those beyond the next leaf, [nx, k1), where the leaf's rows
+// also become U12 = L11^-1 A12.  32 columns per CTA of 4 warps; bound by latency (moves, rows, 32
+// substitution steps), so all loads of a thread are in flight together and four lanes share a column
+// of the substitution.  Runs on the leaf stream under the next leaf, whose time it must not exceed:
+// leaf_swap_u12_kernel took 16 us for each side (it composes the interchanges itself, 3.7 us, and a
+// thread owns a whole column), this takes 5.7 us for both.
+constexpr int kLsThreads = 128;
+__global__ void __launch_bounds__(kLsThreads) leaf_side_kernel(double* A, int64_t ld, int c0, int w, int k0, int nx,
+                                                               int k1, const int32_t* moves, int32_t* perm,
+                                                               int32_t* pmap, const int32_t* status) {
+    __shared__ double s_x[kPanelW][kPanelW + 1], s_e[kPanelW][kPanelW + 1], s_l[kPanelW][kPanelW + 1];
+    __shared__ int s_mv[3 * kPanelW + 1];
+    if (status[kInfo] != 0) return;
+    const int t = threadIdx.x, lane = t & 31, wp = t >> 5;
+    const int nleft = (c0 - k0 + kPanelW - 1) / kPanelW;
+    const bool right = (int)blockIdx.x >= nleft;
+    const int cb = right ? nx + ((int)blockIdx.x - nleft) * kPanelW : k0 + (int)blockIdx.x * kPanelW;
+    const int col = cb + lane, end = right ? k1 : c0;
+    double l[kPanelW * kPanelW / kLsThreads];  // L11 (rows wp + 4 i, column `lane`)
+#pragma unroll
+    for (int i = 0; i < kPanelW / 4; ++i) {
+        const int j = wp + 4 * i;
+        l[i] = (right && j < w && lane < j) ? A[(int64_t)(c0 + j) * ld + c0 + lane] : 0.0;
+    }
+    if (t < 3 * kPanelW + 1) s_mv[t] = moves[t];
+    __syncthreads();
+    const int nx_rows = s_mv[kPanelW];
+    double x[kPanelW / 4], e[kPanelW / 4];
+#pragma unroll
+    for (int i = 0; i < kPanelW / 4; ++i) {
+        const int j = wp + 4 * i;
+        x[i] = (col < end && j < w) ? A[(int64_t)s_mv[j] * ld + col] : 0.0;
+        e[i] = (col < end && j < nx_rows) ? A[(int64_t)s_mv[2 * kPanelW + 1 + j] * ld + col] : 0.0;
+    }
+    int pv = 0, qv = 0, dst = -1;  // the maps: thread t < 32 the leaf's rows, t < 64 the others
+    if (blockIdx.x == 0 && t < 2 * kPanelW) {
+        const bool top = t < kPanelW;
+        const int j = top ? t : t - kPanelW;
+        if (top ? j < w : j < nx_rows) {
+            const int src = s_mv[top ? j : 2 * kPanelW + 1 + j];
+            dst = top ? c0 + j : s_mv[kPanelW + 1 + j];
+            if (perm) pv = perm[src];
+            if (pmap) qv = pmap[src];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kPanelW / 4; ++i) {
+        s_x[wp + 4 * i][lane] = x[i];
+        s_e[wp + 4 * i][lane] = e[i];
+        s_l[wp + 4 * i][lane] = l[i];
+    }
+    __syncthreads();  // every source of these columns, and of the maps, has been read
+    if (dst >= 0) {
+        if (perm) perm[dst] = pv;
+        if (pmap) pmap[dst] = qv;
+    }
+    if (right) {
+        // warp = 8 columns, lane = column + 8 * (row & 3); four rows a step, the finished element
+        // broadcast by a shuffle; contributions in ascending order
+        const int c = 8 * wp + (lane & 7), rg = lane >> 3;
+#pragma unroll
+        for (int i = 0; i < kPanelW / 4; ++i) x[i] = s_x[4 * i + rg][c];
+#pragma unroll 1
+        for (int q = 0; q < kPanelW / 4; ++q) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const double xi = __shfl_sync(0xffffffffu, x[0], (lane & 7) + 8 * u);
+                const double* lt = &s_l[4 * q + rg][4 * q + u];
+                if (rg > u) x[0] = fma(-lt[0], xi, x[0]);
+#pragma unroll
+                for (int i = 1; i < kPanelW / 4; ++i)
+                    if (q + i < kPanelW / 4) x[i] = fma(-lt[4 * i * (kPanelW + 1)], xi, x[i]);
+            }
+            s_x[4 * q + rg][c] = x[0];
+#pragma unroll
+            for (int i = 1; i < kPanelW / 4; ++i) x[i - 1] = x[i];
+        }
+        __syncthreads();
+    }
+    if (col < end) {
+#pragma unroll
+        for (int i = 0; i < kPanelW / 4; ++i) {
+            const int j = wp + 4 * i;
+            if (j < w && (right || s_mv[j] != c0 + j)) A[(int64_t)(c0 + j) * ld + col] = s_x[j][lane];
+            if (j < nx_rows) A[(int64_t)s_mv[kPanelW + 1 + j] * ld + col] = s_e[j][lane];
+        }
+    }
+}
+
 // A[r][c] -= sum_{k < w} A[r][c0 + k] * A[c0 + k][c] for rows [r_lo, n) and columns [cl, ch): the
 // leaf's rank-w update of the rest of its outer panel.  64 x 64 tiles, 4 x 4 per thread, the
 // L21 and U12 slices staged in shared memory; the w products of each element are accumulated in
@@ -339,44 +429,50 @@ __global__ void __launch_bounds__(256, 2) panel_rank_update_kernel(double* A, in
 }
 
 // U12 = L11^-1 A12 for one outer panel in a single launch: L11 unit lower (k <= 256 rows, at L with
-// row stride ldl), the right-hand sides k x ncols at B.  A CTA owns 32 columns, held in shared
-// memory for the whole solve; per 32-row block of L11 (staged in shared memory by cp.async, the
-// next block column while the current one is used): warp 0 substitutes the block's diagonal
-// triangle (lane = column; contributions in ascending order, as trsm_small_kernel computes them),
-// then every warp subtracts the block's contribution from the rows below it (each element's 32
-// products accumulated in ascending order and subtracted once).
+// row stride ldl), the right-hand sides k x ncols at B.  A CTA owns NC columns, held in shared memory
+// for the whole solve; per 32-row block of L11 (its block column staged by cp.async, the next one
+// while the current one is used) one warp per 8 columns substitutes the block's triangle, four lanes
+// a column (contributions in ascending order), and all warps subtract the block's contribution from
+// the rows below it on the FP64 tensor cores.  What bounds it is the chain of the eight blocks, so
+// the columns of the next panel, which are on the critical path, run eight to a CTA (32 CTAs for 256
+// columns), and only right-hand sides beyond what one wave holds so run 32 to a CTA, which reads L11
+// a quarter as often.  256 rows, 256 columns: 60 us before (32 columns a CTA, one warp substituting a
+// 32 x 32 triangle from unrolled code), 25.6 us with 8 columns a CTA, 39 us with 32.
 constexpr int kTpK = 256;   // rows of the panel
-constexpr int kTpC = 32;    // columns per CTA
-constexpr int kTpSmem = (kTpK * kTpC + 2 * kTpK * kPanelW) * (int)sizeof(double);  // 192 KiB
+constexpr int kTpThreads = 256;
+constexpr int kTpPitch = kTpK + 4;  // columns of X in shared memory (column-major; conflict-free fragments)
+template <int NC> constexpr int tp_smem() { return (NC * kTpPitch + 2 * kTpK * kPanelW) * (int)sizeof(double); }
 
-__global__ void __launch_bounds__(256, 1) trsm_panel_kernel(const double* L, int64_t ldl, double* B, int64_t ldb,
-                                                            int k, int ncols, const int32_t* status) {
+template <int NC>
+__global__ void __launch_bounds__(kTpThreads, 1) trsm_panel_kernel(const double* L, int64_t ldl, double* B,
+                                                                   int64_t ldb, int k, int ncols,
+                                                                   const int32_t* status) {
     extern __shared__ __align__(16) double tp_dyn[];
-    double* s_x = tp_dyn;                         // [kTpK][kTpC] this CTA's columns
-    double* s_l = tp_dyn + kTpK * kTpC;           // [2][kTpK][kPanelW] block columns of L11 (rows 32 i ..)
+    double* s_l = tp_dyn;                         // [2][kTpK][kPanelW] block columns of L11, pairs swizzled by row
+    double* s_x = tp_dyn + 2 * kTpK * kPanelW;    // [NC][kTpPitch] this CTA's columns (zero past row k)
+    __shared__ double s_t[kPanelW][kPanelW + 1];  // the block's triangle
     if (status[kInfo] != 0) return;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int cb = blockIdx.x * kTpC;
+    const int cb = blockIdx.x * NC;
     const int nb = (int)ceil_div(k, kPanelW);
+    auto sx = [](int row, int c) { return row * kPanelW + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
     // block column i of L11: rows [32 i, k), columns [32 i, 32 i + 32) -> buffer i & 1 (16-byte pieces)
     auto stage = [&](int i) {
         double* dst = s_l + (i & 1) * kTpK * kPanelW;
-        const int r0 = kPanelW * i, rows = k - r0;
-        for (int e = t; e < rows * (kPanelW / 2); e += 256) {
-            const int rr = e / (kPanelW / 2), q2 = e - rr * (kPanelW / 2);
-            const int col = r0 + 2 * q2;
-            const double* src = L + (int64_t)(r0 + rr) * ldl + col;
-            cp_async16(dst + rr * kPanelW + 2 * q2, src, col + 1 < k ? 16 : (col < k ? 8 : 0));
-        }
+        const int r0 = kPanelW * i, c = 2 * (t & 15), col = r0 + c;
+        const int bytes = col + 1 < k ? 16 : (col < k ? 8 : 0);
+        const double* src = L + (int64_t)r0 * ldl + (col < k ? col : 0);
+#pragma unroll 4
+        for (int r = t >> 4; r < k - r0; r += kTpThreads / 16) cp_async16(dst + sx(r, c), src + (int64_t)r * ldl, bytes);
         cp_async_commit();
     };
     stage(0);
-    batched_copy<256, 8, double>(t, kTpK * kTpC,
+    batched_copy<kTpThreads, 8, double>(t, kTpK * NC,
         [&](int e) {
-            const int r = e / kTpC, c = e - r * kTpC;
+            const int r = e / NC, c = e % NC;
             return (r < k && cb + c < ncols) ? B[(int64_t)r * ldb + cb + c] : 0.0;
         },
-        [&](int e, double v) { s_x[e] = v; });
+        [&](int e, double v) { s_x[(e % NC) * kTpPitch + e / NC] = v; });
     for (int i = 0; i < nb; ++i) {
         if (i + 1 < nb) {
             stage(i + 1);
@@ -385,43 +481,64 @@ __global__ void __launch_bounds__(256, 1) trsm_panel_kernel(const double* L, int
             cp_async_wait<0>();
         }
         __syncthreads();
-        const double* lb = s_l + (i & 1) * kTpK * kPanelW;  // lb[(r - 32 i) * 32 + q] = L[r][32 i + q]
+        const double* lb = s_l + (i & 1) * kTpK * kPanelW;  // lb[sx(r - 32 i, q)] = L[r][32 i + q]
         const int r0 = kPanelW * i, bw = min(kPanelW, k - r0);
-        if (warp == 0) {
-            double x[kPanelW];
-#pragma unroll
-            for (int j = 0; j < kPanelW; ++j) x[j] = s_x[(r0 + min(j, bw - 1)) * kTpC + lane];
-#pragma unroll
-            for (int q = 0; q < kPanelW - 1; ++q) {
-#pragma unroll
-                for (int j = q + 1; j < kPanelW; ++j)
-                    if (j < bw) x[j] = fma(-lb[j * kPanelW + q], x[q], x[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < kPanelW; ++j)
-                if (j < bw) s_x[(r0 + j) * kTpC + lane] = x[j];
+        for (int e = t; e < kPanelW * kPanelW; e += kTpThreads) {  // the triangle, for constant offsets below
+            const int r = e >> 5, c = e & 31;
+            s_t[r][c] = (r < bw && c < r) ? lb[sx(r, c)] : 0.0;
         }
         __syncthreads();
-        // rows below the block: thread (warp, lane) updates rows r0 + bw + warp + 8 m of column lane
-        double xb[kPanelW];
+        if (warp < NC / 8) {
+            // warp = 8 columns, lane = column + 8 * (row & 3); rows past the end are zero and stay so
+            double* xc = s_x + (8 * warp + (lane & 7)) * kTpPitch + r0;
+            const int rg = lane >> 3;
+            double x[kPanelW / 4];
 #pragma unroll
-        for (int q = 0; q < kPanelW; ++q) xb[q] = q < bw ? s_x[(r0 + q) * kTpC + lane] : 0.0;
-        for (int r = r0 + bw + warp; r < k; r += 8) {
-            const double* lr = lb + (r - r0) * kPanelW;
-            double acc = 0.0;
+            for (int e = 0; e < kPanelW / 4; ++e) x[e] = xc[4 * e + rg];
+            const double* lt = &s_t[rg][0];
+#pragma unroll 1
+            for (int q = 0; q < kPanelW / 4; ++q, lt += 4 * (kPanelW + 1) + 4) {
 #pragma unroll
-            for (int q = 0; q < kPanelW; q += 2) {
-                const double2 l2 = *reinterpret_cast<const double2*>(lr + q);
-                acc = fma(l2.x, xb[q], acc);
-                acc = fma(l2.y, xb[q + 1], acc);
+                for (int u = 0; u < 4; ++u) {
+                    const double xi = __shfl_sync(0xffffffffu, x[0], (lane & 7) + 8 * u);
+                    if (rg > u) x[0] = fma(-lt[u], xi, x[0]);
+#pragma unroll
+                    for (int e = 1; e < kPanelW / 4; ++e)
+                        if (q + e < kPanelW / 4) x[e] = fma(-lt[4 * e * (kPanelW + 1) + u], xi, x[e]);
+                }
+                xc[4 * q + rg] = x[0];
+#pragma unroll
+                for (int e = 1; e < kPanelW / 4; ++e) x[e - 1] = x[e];
             }
-            s_x[r * kTpC + lane] -= acc;
+        }
+        __syncthreads();
+        // rows below the block (only full blocks have any), 16 x 8 tiles:
+        // a = L[g][k + tq], L[g + 8][k + tq], b = x[k + tq][g], c = rows g, g + 8, columns 2 tq, 2 tq + 1
+        const int g = lane >> 2, tq = lane & 3;
+        const int mt = (k - r0 - bw + 15) / 16;
+        for (int tile = warp; tile < mt * (NC / 8); tile += kTpThreads / 32) {
+            const int c8 = 8 * (tile % (NC / 8)), ra = bw + 16 * (tile / (NC / 8)) + g, rb = ra + 8;
+            const bool oka = r0 + ra < k, okb = r0 + rb < k;
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            const double* xb = s_x + (c8 + g) * kTpPitch + r0 + tq;
+#pragma unroll
+            for (int q = 0; q < kPanelW / 4; ++q) {
+                const double a0 = oka ? lb[sx(ra, 4 * q + tq)] : 0.0, a1 = okb ? lb[sx(rb, 4 * q + tq)] : 0.0;
+                const double b0 = xb[4 * q];
+                asm volatile(
+                    "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+                    : "+d"(acc[0]), "+d"(acc[1]), "+d"(acc[2]), "+d"(acc[3])
+                    : "d"(a0), "d"(a1), "d"(b0));
+            }
+            double* xd = s_x + (c8 + 2 * tq) * kTpPitch + r0;
+            if (oka) { xd[ra] -= acc[0]; xd[kTpPitch + ra] -= acc[1]; }
+            if (okb) { xd[rb] -= acc[2]; xd[kTpPitch + rb] -= acc[3]; }
         }
         __syncthreads();  // the buffer of block i is restaged for block i + 2
     }
-    for (int e = t; e < kTpK * kTpC; e += 256) {
-        const int r = e / kTpC, c = e - r * kTpC;
-        if (r < k && cb + c < ncols) B[(int64_t)r * ldb + cb + c] = s_x[e];
+    for (int e = t; e < kTpK * NC; e += kTpThreads) {
+        const int r = e / NC, c = e % NC;
+        if (r < k && cb + c < ncols) B[(int64_t)r * ldb + cb + c] = s_x[c * kTpPitch + r];
     }
 }
 
@@ -550,26 +667,109 @@ __global__ void gather_rows_kernel(double* X, int64_t ldx, const double* B, int6
     X[i * ldx + c] = B[(int64_t)perm[i] * ldb + c];
 }
 
-// perm from a LAPACK-style ipiv: sequential interchanges, on a shared-memory copy when `in_smem`
-// (n ints fit), else directly in perm (global memory; one dependent swap per step)
-__global__ void perm_from_ipiv_kernel(const int32_t* ipiv, int n, int32_t* perm, int in_smem) {
-    extern __shared__ int32_t pv_dyn[];
-    int32_t* pv = in_smem ? pv_dyn : perm;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) pv[i] = i;
+// perm from a LAPACK-style ipiv: the result of the sequential interchanges of 0, 1, 2, ...
+//
+// Where every interchange reaches forward (i <= ipiv[i] < n or out of range, which means none), the
+// content a position has at a step follows from the last earlier interchange that reached it: with
+// V(j) the content of position j before step j,
+//     V(j) = V(k), k the last k < j with ipiv[k] = j, or j if there is none;
+//     perm[i] = V(i) if ipiv[i] = i, else V(k), k the last k < i with ipiv[k] = ipiv[i], or ipiv[i].
+// The first k is a maximum over all interchanges; the second comes from one warp walking the steps 32
+// at a time with a table of the last interchange per position; V by pointer jumping.  One thread's
+// sequential interchanges (140 cycles each) remain for other vectors and orders: order 4096 took
+// 283 us, now
+// 37.
+constexpr int kPermThreads = 1024;
+constexpr uint16_t kPermNone = 0xffff;
+constexpr int kPermMax = 32768;  // orders whose three tables of 16-bit indices fit shared memory
+__global__ void __launch_bounds__(kPermThreads) perm_from_ipiv_kernel(const int32_t* ipiv, int n, int32_t* perm) {
+    extern __shared__ __align__(16) uint16_t pi_dyn[];
+    uint16_t* up = pi_dyn;            // the targets; then V's pointers: up[j] = the k of V(j), or j
+    uint16_t* last = pi_dyn + n;      // position -> last interchange that reached it so far
+    uint16_t* prev = pi_dyn + 2 * n;  // i -> the last k < i with ipiv[k] = ipiv[i]
+    __shared__ int s_back;
+    const int t = threadIdx.x, lane = t & 31;
+    auto target = [&](int i) {
+        const int q = ipiv[i];
+        return q >= 0 && q < n ? q : i;
+    };
+    if (t == 0) s_back = 0;
+    __syncthreads();
+    for (int i = t; i < n; i += kPermThreads) {
+        const int q = target(i);
+        up[i] = (uint16_t)q;
+        last[i] = kPermNone;
+        if (q < i) s_back = 1;
+    }
+    __syncthreads();
+    if (s_back) {  // an interchange that reaches back: step by step, `last` as the permutation
+        for (int i = t; i < n; i += kPermThreads) last[i] = (uint16_t)i;
+        __syncthreads();
+        if (t == 0)
+            for (int i = 0; i < n; ++i) {
+                const int q = up[i];
+                const uint16_t v = last[i];
+                last[i] = last[q];
+                last[q] = v;
+            }
+        __syncthreads();
+        for (int i = t; i < n; i += kPermThreads) perm[i] = last[i];
+        return;
+    }
+    if (t < 32) {
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const int i = i0 + lane, q = i < n ? up[i] : -1 - lane;
+            const uint32_t same = __match_any_sync(0xffffffffu, q);
+            const uint32_t before = same & ((1u << lane) - 1u);
+            if (i < n) prev[i] = before ? (uint16_t)(i0 + 31 - __clz(before)) : last[q];
+            __syncwarp();
+            if (i < n && (same >> lane) == 1u) last[q] = (uint16_t)i;  // the chunk's last one
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    // `last` now holds, per position, its last interchange of all: of its own step (none before) or
+    // the last earlier one; a position's own step that moves nothing hides the earlier one
+    for (int j = t; j < n; j += kPermThreads) {
+        uint16_t k = last[j];
+        if (k == (uint16_t)j) k = prev[j];
+        up[j] = k != kPermNone ? k : (uint16_t)j;
+    }
+    __syncthreads();
+    // up[j] -> the root of j's chain: every value ever read is one of j's ancestors, so the threads need
+    // not agree on a round's old and new values, and a round in which nothing moved ends it
+    volatile uint16_t* vup = up;
+    for (;;) {
+        int moved = 0;
+        for (int j = t; j < n; j += kPermThreads) {
+            const uint16_t u = vup[j], v = vup[u];
+            if (v != u) {
+                vup[j] = v;
+                moved = 1;
+            }
+        }
+        if (!__syncthreads_or(moved)) break;
+    }
+    for (int i = t; i < n; i += kPermThreads) {
+        const int q = target(i);
+        perm[i] = q == i ? up[i] : (prev[i] != kPermNone ? up[prev[i]] : q);
+    }
+}
+
+// the same for larger orders, step by step in global memory
+__global__ void perm_from_ipiv_serial_kernel(const int32_t* ipiv, int n, int32_t* perm) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = i;
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int i = 0; i < n; ++i) {
             const int q = ipiv[i];
             if (q != i && q >= 0 && q < n) {
-                const int t = pv[i];
-                pv[i] = pv[q];
-                pv[q] = t;
+                const int t = perm[i];
+                perm[i] = perm[q];
+                perm[q] = t;
             }
         }
     }
-    __syncthreads();
-    if (in_smem)
-        for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = pv[i];
 }
 
 // det = (-1)^{#i: ipiv[i] != i} * U[0][0] * U[1][1] * ... in this order (MatrixDeterminant :467-476);
@@ -738,6 +938,8 @@ static_assert(kOuterNB == kTpK, "the panel triangular solve holds one outer pane
 // device factors the first panel while the host submits the second).
 int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, int32_t* ipiv, int32_t* perm,
                    int32_t* pmap2, int64_t leaf, int part) {
+    const bool linked = leaf == kPanelW;  // (the narrower leaves of taller matrices are not linked)
+    int32_t* moves = pmap2 + 2 * round_up(n, 64);
     cudaStream_t q2 = ctx->side_stream;
     bool side_busy = false;
     auto join = [&]() -> int32_t {
@@ -755,9 +957,12 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
     };
     const int64_t pm_ld = round_up(n, 64);
     PriorityScope hi(ctx, true);  // this stream's launches are the critical path (see launch_k)
-    std::atomic<int>& attr = device_flag((const void*)trsm_panel_kernel, 0, ctx->device);
+    std::atomic<int>& attr = device_flag((const void*)trsm_panel_kernel<8>, 0, ctx->device);
     if (!attr.load()) {
-        B2M_CU(ctx, cudaFuncSetAttribute(trsm_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTpSmem));
+        B2M_CU(ctx, cudaFuncSetAttribute(trsm_panel_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         tp_smem<8>()));
+        B2M_CU(ctx, cudaFuncSetAttribute(trsm_panel_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         tp_smem<32>()));
         attr.store(1);
     }
     for (int64_t k0 = 0; k0 < n; k0 += kOuterNB) {
@@ -769,8 +974,8 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
             B2M_LAUNCHED(ctx);
         }
         // The panel, right-looking by leaves.  The critical path, on this stream: a leaf's panel
-        // kernel, then its interchanges, U12 and rank-w update on the next leaf's columns only; the
-        // same for the other columns of the outer panel (the factored ones left of the leaf get the
+        // kernel, then its interchanges, U12 and rank-w update on the next leaf's columns only (in the
+        // next leaf's own kernel when the leaves are linked); the same for the other columns of the outer panel (the factored ones left of the leaf get the
         // interchanges only) runs on the leaf stream, under the next leaf's panel kernel, and is
         // waited for before that leaf's own updates touch those columns.  Column groups are
         // disjoint between the two streams, and every column sees the leaves' interchanges and
@@ -804,21 +1009,41 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
         };
         for (int64_t c0 = k0; leaves && c0 < k1; c0 += leaf) {
             const int64_t wl = std::min(leaf, k1 - c0);
-            B2M_TRY(launch_panel<double>(ctx, q, A + c0 * ld + c0, ld, (int)(n - c0), (int)wl, (int)c0, (int)c0, ipiv));
+            // a linked leaf applies the leaf before it to its own columns; the leaf stream does it for
+            // the rest of the panel and keeps the maps
+            int32_t* mv = moves + kPanelMoves * (c0 / kPanelW & 1);
+            PanelLink link;
+            if (linked && c0 > k0) link.moves_in = moves + kPanelMoves * ((c0 / kPanelW - 1) & 1);
+            if (linked) link.moves_out = mv;
+            B2M_TRY(launch_panel<double>(ctx, q, A + c0 * ld + c0, ld, (int)(n - c0), (int)wl, (int)c0, (int)c0, ipiv,
+                                         link));
             const int64_t rl = c0 + wl, nx = std::min(rl + leaf, k1);  // the next leaf: columns [rl, nx)
             B2M_CU(ctx, cudaEventRecord(ctx->ev_leaf_panel, q));
             if (leaf_busy) {  // the previous leaf's updates of [rl, k1) are done
                 B2M_CU(ctx, cudaStreamWaitEvent(q, ctx->ev_leaf_side, 0));
                 leaf_busy = false;
             }
-            B2M_TRY(swap_u12(q, c0, wl, rl, nx, true));
-            B2M_TRY(rank_update(q, c0, wl, rl, nx, 1 << 30));
-            if (nx < k1 || c0 > k0) {
+            if (!linked) {
+                B2M_TRY(swap_u12(q, c0, wl, rl, nx, true));
+                B2M_TRY(rank_update(q, c0, wl, rl, nx, 1 << 30));
+            }
+            if (nx < k1 || c0 > k0 || linked) {
                 PriorityScope side(ctx, false);
                 B2M_CU(ctx, cudaStreamWaitEvent(ql, ctx->ev_leaf_panel, 0));
-                B2M_TRY(swap_u12(ql, c0, wl, nx, k1, false));
-                B2M_TRY(swap_u12(ql, c0, wl, k0, c0, false));
-                B2M_TRY(rank_update(ql, c0, wl, nx, k1, 64));
+                if (linked) {
+                    const int64_t groups = ceil_div(c0 - k0, kPanelW) + ceil_div(k1 - nx, kPanelW);
+                    prof_begin(ctx, ql, kClsSwap);
+                    B2M_CU(ctx, launch_k(ctx, leaf_side_kernel, dim3((unsigned)std::max<int64_t>(1, groups)),
+                                         dim3(kLsThreads), 0, ql, A, ld, (int)c0, (int)wl, (int)k0, (int)nx, (int)k1,
+                                         (const int32_t*)mv, perm, pmap, (const int32_t*)ctx->d_status));
+                    prof_end(ctx, ql, kClsSwap, 16.0 * wl * (double)(k1 - nx + c0 - k0));
+                    B2M_LAUNCHED(ctx);
+                } else {
+                    B2M_TRY(swap_u12(ql, c0, wl, nx, k1, false));
+                    B2M_TRY(swap_u12(ql, c0, wl, k0, c0, false));
+                }
+                // (the next leaf's cluster needs 16 SMs to itself)
+                B2M_TRY(rank_update(ql, c0, wl, nx, k1, linked ? 2 * (ctx->num_sms - 16) : 64));
                 B2M_CU(ctx, cudaEventRecord(ctx->ev_leaf_side, ql));
                 leaf_busy = true;
             }
@@ -854,8 +1079,11 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
         if (k1 >= n) break;
         auto update = [&](cudaStream_t qs, int64_t cs, int64_t nc) -> int32_t {
             prof_begin(ctx, qs, kClsTrsm);
-            B2M_CU(ctx, launch_k(ctx, trsm_panel_kernel, dim3((unsigned)ceil_div(nc, kTpC)), dim3(256), (size_t)kTpSmem,
-                                 qs, (const double*)(A + k0 * ld + k0), ld, A + k0 * ld + cs, ld, (int)w, (int)nc,
+            const bool few = nc <= 8 * ctx->num_sms;
+            B2M_CU(ctx, launch_k(ctx, few ? trsm_panel_kernel<8> : trsm_panel_kernel<32>,
+                                 dim3((unsigned)ceil_div(nc, few ? 8 : 32)), dim3(kTpThreads),
+                                 (size_t)(few ? tp_smem<8>() : tp_smem<32>()), qs,
+                                 (const double*)(A + k0 * ld + k0), ld, A + k0 * ld + cs, ld, (int)w, (int)nc,
                                  (const int32_t*)ctx->d_status));
             prof_end(ctx, qs, kClsTrsm, 8.0 * (w * (double)w / 2 + 2.0 * w * (double)nc));  // bytes
             B2M_LAUNCHED(ctx);
@@ -943,7 +1171,7 @@ int32_t lu_factor_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t 
     int32_t* pmap2 = nullptr;
     if (blocked) {
         void* p = nullptr;
-        B2M_TRY(ws_get(ctx, kWsPmap, (size_t)(2 * round_up(n, 64)) * sizeof(int32_t), &p));
+        B2M_TRY(ws_get(ctx, kWsPmap, (size_t)(2 * round_up(n, 64) + 2 * kPanelMoves) * sizeof(int32_t), &p));
         pmap2 = static_cast<int32_t*>(p);
         B2M_TRY(ensure_side_stream(ctx));
     }
@@ -990,17 +1218,18 @@ int32_t lu_solve_f64(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld, in
 
 int32_t perm_from_ipiv(Ctx* ctx, cudaStream_t st, const int32_t* ipiv, int64_t n, int32_t* perm) {
     if (n > (1 << 30)) return fail(ctx, B2M_ERR_UNSUPPORTED, "perm_from_ipiv: n too large");
-    const size_t smem = (size_t)n * sizeof(int32_t);
-    const bool in_smem = smem <= ctx->smem_optin;
-    if (in_smem && smem > 48 * 1024) {
+    const size_t smem = (size_t)n * 3 * sizeof(uint16_t);
+    if (n <= kPermMax && smem <= ctx->smem_optin) {
         std::atomic<int>& set = device_flag((const void*)perm_from_ipiv_kernel, 0, ctx->device);
         if (!set.load()) {
             B2M_CU(ctx, cudaFuncSetAttribute(perm_from_ipiv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)ctx->smem_optin));
+                                             3 * kPermMax * (int)sizeof(uint16_t)));
             set.store(1);
         }
+        perm_from_ipiv_kernel<<<1, kPermThreads, smem, st>>>(ipiv, (int)n, perm);
+    } else {
+        perm_from_ipiv_serial_kernel<<<1, 1024, 0, st>>>(ipiv, (int)n, perm);
     }
-    perm_from_ipiv_kernel<<<1, 1024, in_smem ? smem : 0, st>>>(ipiv, (int)n, perm, in_smem ? 1 : 0);
     B2M_LAUNCHED(ctx);
     return B2M_OK;
 }

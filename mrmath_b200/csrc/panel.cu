@@ -457,6 +457,18 @@ __device__ __noinline__ int warp_winner(double a, int pos) {
     return __ffs(__ballot_sync(0xffffffffu, top && (uint32_t)pos == mp)) - 1;
 }
 
+// The previous leaf of the same outer panel (PanelLink::moves_in not null): the kernel first applies
+// its interchanges, its triangular solve and its rank-32 update to the leaf's own columns, which still
+// lack them.  As separate launches these were most of what lay between two leaves: 16 us for the
+// interchanges with U12 (7,200 cycles of it composing the interchanges, which the scribe warp now
+// does while the leaf is factored), 9 us for the update, and two launches.  In here they take 5.5 us
+// (1024 and 2048 rows: 31.7 -> 37 us; 512 rows: 28.6 -> 37; 4096 rows: 38 -> 47).
+// Moves: [0, 32) the row whose content ends in each of the leaf's rows, [32] the number of rows below
+// the leaf that receive another row, [33, 65) these rows, [65, 97) the rows they receive.
+constexpr int kPMoves = 3 * kPW + 1;
+constexpr int kPLRows = 256;             // rows of L21 staged at a time
+constexpr int kPLtPitch = kPW + 1;
+
 // a warp's candidate for the pivot of a column
 struct __align__(16) PCand {
     double rinv;       // 1 / row[0]
@@ -471,7 +483,7 @@ __device__ __forceinline__ int cand_pieces(int col) { return 1 + (kPBk + 1 - (co
 template <int RPT, bool MULTI>
 __global__ void __launch_bounds__(kPNa, 1)
     panel_kernel(double* P, int64_t ld, int m, int w, int R, int row_base, int col_base, int32_t* ipiv,
-                 int32_t* status) {
+                 int32_t* status, PanelLink link) {
     int C = 1, rank = 0;
     if constexpr (MULTI) {
         C = (int)cg::this_cluster().num_blocks();
@@ -489,6 +501,15 @@ __global__ void __launch_bounds__(kPNa, 1)
     __shared__ __align__(16) double s_l[kPBk][kPBk];        // the block's rows of L11
     __shared__ __align__(8) uint64_t s_bar[kPSlots], s_rbar;    // a column's candidates; a block's pivot rows
     __shared__ int s_pl[kPW], s_ps[kPW];                        // the pivots: local row, CTA
+    __shared__ int s_mv[kPMoves];
+    // Staging of the previous leaf's L21 rows (s_ll) and of its L11, then U12 (s_lt).  In a cluster it
+    // lies in s_rcv: slot 0 may be written by CTAs that are done with their prologue, slots 1 .. 13
+    // hold s_ll (no candidate of column 1 is sent before every CTA has sent column 0), the last two
+    // s_lt (not written before the scribe has left column 7).
+    double* s_ll = MULTI ? reinterpret_cast<double*>(&s_rcv[1][0]) : S + (size_t)kPW * R;
+    double* s_lt = MULTI ? reinterpret_cast<double*>(&s_rcv[kPSlots - 2][0]) : s_ll + kPW * kPLRows;
+    static_assert(sizeof(PCand) * kPNw * kPMaxC * (kPSlots - 3) >= sizeof(double) * kPW * kPLRows, "s_ll fits");
+    static_assert(sizeof(PCand) * kPNw * kPMaxC * 2 >= sizeof(double) * kPW * kPLtPitch, "s_lt fits");
     if (status[kInfo] != 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int lo = rank * R;
@@ -509,15 +530,121 @@ __global__ void __launch_bounds__(kPNa, 1)
         __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
     }
+    const bool linked = link.moves_in != nullptr;
     {
         constexpr int RS = kPNa / (kPW / 2);  // rows per step
         const int c = 2 * (tid % (kPW / 2));
-        const int bytes = c + 1 < w ? 16 : (c < w ? 8 : 0);
-        const double* src = P + (int64_t)(lo + tid / (kPW / 2)) * ld + (c < w ? c : 0);
+        const int bytes = c + 1 < w ? 16 : (c < w ? 8 : 0), cc = c < w ? c : 0;
+        if (!linked) {
+            const double* src = P + (int64_t)(lo + tid / (kPW / 2)) * ld + cc;
 #pragma unroll 4
-        for (int rl = tid / (kPW / 2); rl < nr; rl += RS, src += RS * ld) cp_async16(S + sx(rl, c), src, bytes);
+            for (int rl = tid / (kPW / 2); rl < nr; rl += RS, src += RS * ld) cp_async16(S + sx(rl, c), src, bytes);
+            cp_async_commit();
+        } else {
+            // the rows as the previous leaf's interchanges leave them, its top rows (positions -32 .. -1
+            // here) and its L11 first, then this CTA's rows and their multipliers
+            int* s_map = reinterpret_cast<int*>(&s_loc[0][0]);
+            static_assert(sizeof(s_loc) >= (size_t)kPNt * RPT * sizeof(int), "the row map fits");
+            const int mv = tid < kPMoves ? link.moves_in[tid] : 0;  // (fewer moves than threads)
+            for (int rl = tid; rl < nr; rl += kPNa) s_map[rl] = lo + rl;
+            if (tid < kPMoves) s_mv[tid] = mv;
+            __syncthreads();
+            if (tid < s_mv[kPW]) {
+                const int d = s_mv[kPW + 1 + tid] - row_base - lo;
+                if (d >= 0 && d < nr) s_map[d] = s_mv[2 * kPW + 1 + tid] - row_base;
+            }
+            for (int rl = tid / (kPW / 2); rl < kPW; rl += RS)
+                cp_async16(&s_u[rl][c], P + (int64_t)(s_mv[rl] - row_base) * ld + cc, bytes);
+            for (int e = tid; e < kPW * kPW; e += kPNa)
+                cp_async8(s_lt + (e >> 5) * kPLtPitch + (e & 31), P + (int64_t)((e >> 5) - kPW) * ld + (e & 31) - kPW, 8);
+            cp_async_commit();
+            __syncthreads();
+#pragma unroll 4
+            for (int rl = tid / (kPW / 2); rl < nr; rl += RS)
+                cp_async16(S + sx(rl, c), P + (int64_t)s_map[rl] * ld + cc, bytes);
+            const double* src = P + (int64_t)(lo + tid / (kPW / 2)) * ld + c - kPW;
+#pragma unroll 4
+            for (int rl = tid / (kPW / 2); rl < min(nr, kPLRows); rl += RS, src += RS * ld)
+                cp_async16(s_ll + sx(rl, c), src, 16);
+            cp_async_commit();
+            cp_async_wait<1>();
+            __syncthreads();
+            if (warp < kPNw) {
+                // U12 = L11^-1 (top rows): warp = 8 columns, lane = column + 8 * (row & 3); four rows a
+                // step, the finished element broadcast by a shuffle; contributions in ascending order
+                const int col = 8 * warp + (lane & 7), rg = lane >> 3;
+                double x[kPW / 4];
+#pragma unroll
+                for (int i = 0; i < kPW / 4; ++i) x[i] = s_u[4 * i + rg][col];
+#pragma unroll 1
+                for (int q = 0; q < kPW / 4; ++q) {
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) {
+                        const double xi = __shfl_sync(0xffffffffu, x[0], (lane & 7) + 8 * t);
+                        const double* lt = s_lt + (4 * q + rg) * kPLtPitch + 4 * q + t;
+                        if (rg > t) x[0] = fma(-lt[0], xi, x[0]);
+#pragma unroll
+                        for (int i = 1; i < kPW / 4; ++i)
+                            if (q + i < kPW / 4) x[i] = fma(-lt[4 * i * kPLtPitch], xi, x[i]);
+                    }
+                    s_u[4 * q + rg][col] = x[0];
+#pragma unroll
+                    for (int i = 1; i < kPW / 4; ++i) x[i - 1] = x[i];
+                }
+            }
+            cp_async_wait<0>();
+            __syncthreads();
+            // rows -= L21 U12 on the FP64 tensor cores, 16 rows a step; U12's fragments stay in registers
+            // (a = L21[g][k + t], L21[g + 8][k + t], b = U12[k + t][g], c = rows g, g + 8, columns 2t, 2t + 1)
+            if (warp < kPNw) {
+                const int g = lane >> 2, t = lane & 3;
+                double bf[kPW / 4][kPW / 8];
+#pragma unroll
+                for (int k = 0; k < kPW / 4; ++k)
+#pragma unroll
+                    for (int j = 0; j < kPW / 8; ++j) bf[k][j] = s_u[4 * k + t][8 * j + g];
+                for (int ch = 0; ch < nr; ch += kPLRows) {
+                    if (ch > 0) {  // the next rows' multipliers take the place of the last ones
+                        asm volatile("bar.sync 3, %0;\n" ::"n"(kPNt) : "memory");
+                        constexpr int RM = kPNt / (kPW / 2);
+#pragma unroll 4
+                        for (int rl = ch + tid / (kPW / 2); rl < min(nr, ch + kPLRows); rl += RM)
+                            cp_async16(s_ll + sx(rl - ch, c), P + (int64_t)(lo + rl) * ld + c - kPW, 16);
+                        cp_async_commit();
+                        cp_async_wait<0>();
+                        asm volatile("bar.sync 3, %0;\n" ::"n"(kPNt) : "memory");
+                    }
+#pragma unroll 1
+                    for (int r0 = ch + 16 * warp; r0 < min(nr, ch + kPLRows); r0 += 16 * kPNw) {
+                        const int ra = r0 + g, rb = ra + 8;
+                        const bool oka = ra < nr, okb = rb < nr;
+                        double acc[kPW / 8][4] = {};
+#pragma unroll
+                        for (int k = 0; k < kPW / 4; ++k) {
+                            const double a0 = oka ? s_ll[sx(ra - ch, 4 * k + t)] : 0.0;
+                            const double a1 = okb ? s_ll[sx(rb - ch, 4 * k + t)] : 0.0;
+#pragma unroll
+                            for (int j = 0; j < kPW / 8; ++j)
+                                asm volatile(
+                                    "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+                                    "{%0,%1,%2,%3};\n"
+                                    : "+d"(acc[j][0]), "+d"(acc[j][1]), "+d"(acc[j][2]), "+d"(acc[j][3])
+                                    : "d"(a0), "d"(a1), "d"(bf[k][j]));
+                        }
+#pragma unroll
+                        for (int j = 0; j < kPW / 8; ++j) {
+                            double2* pa = reinterpret_cast<double2*>(S + sx(ra, 8 * j + 2 * t));
+                            double2* pb = reinterpret_cast<double2*>(S + sx(rb, 8 * j + 2 * t));
+                            if (oka) *pa = make_double2(pa->x - acc[j][0], pa->y - acc[j][1]);
+                            if (okb) *pb = make_double2(pb->x - acc[j][2], pb->y - acc[j][3]);
+                        }
+                    }
+                }
+                // U12 out of the way of this leaf's U (L11 is no longer read)
+                for (int e = tid; e < kPW * kPW; e += kPNt) s_lt[(e >> 5) * kPLtPitch + (e & 31)] = s_u[e >> 5][e & 31];
+            }
+        }
     }
-    cp_async_commit();
     cp_async_wait<0>();
     __syncthreads();
     if constexpr (MULTI) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
@@ -593,6 +720,11 @@ __global__ void __launch_bounds__(kPNa, 1)
     bool stop = false;
     if (warp == kPNw) {
         // ---- scribe warp: records each pivot, and the pivot row's part of U inside its block
+        // It also composes the interchanges into moves: lane i holds the position whose content ends in
+        // position i (sm), lane e < n_extra a position below the leaf that an interchange reached and
+        // the one whose content ends there.
+        int sm = lane, my_pos = -1, my_src = -1, n_extra = 0;
+        bool done = true;
         for (int j = 0; j < w; ++j) {
             if constexpr (MULTI) {
                 wait_col(j);
@@ -602,7 +734,31 @@ __global__ void __launch_bounds__(kPNa, 1)
             int win;
             const PCand* b = select(j, win);
             const double v = lane < kPBk ? b->row[lane] : 0.0;
-            if (!(fabs(b->row[0]) > sing_thresh<double>())) break;
+            if (!(fabs(b->row[0]) > sing_thresh<double>())) {
+                done = false;
+                break;
+            }
+            if (j == 0 && linked && rank == 0 && !late) {
+                // every CTA has read its rows: U12 of the previous leaf takes its place
+#pragma unroll 8
+                for (int r = 0; r < kPW; ++r)
+                    if (lane < w) P[(int64_t)(r - kPW) * ld + lane] = s_lt[r * kPLtPitch + lane];
+            }
+            {
+                const int q = b->pos, a = __shfl_sync(0xffffffffu, sm, j);
+                int other;
+                if (q < w) {
+                    other = __shfl_sync(0xffffffffu, sm, q);
+                    if (lane == q) sm = a;
+                } else {
+                    const uint32_t hit = __ballot_sync(0xffffffffu, my_pos == q);
+                    const int e = hit ? __ffs(hit) - 1 : n_extra++;
+                    if (!hit && lane == e) my_pos = my_src = q;
+                    other = __shfl_sync(0xffffffffu, my_src, e);
+                    if (lane == e) my_src = a;
+                }
+                if (lane == j) sm = other;
+            }
             if (lane < kPBk && (j & (kPBk - 1)) + lane < kPBk && j + lane < kPW) s_u[j][j + lane] = v;
             if (lane == 0) {
                 if (rank == 0) ipiv[col_base + j] = row_base + b->pos;
@@ -615,6 +771,12 @@ __global__ void __launch_bounds__(kPNa, 1)
             } else if (j + 1 == w) {
                 asm volatile("bar.sync 2, %0;\n" ::"r"(kPNa) : "memory");
             }
+        }
+        if (done && rank == 0 && link.moves_out) {
+            link.moves_out[lane] = row_base + sm;
+            if (lane == 0) link.moves_out[kPW] = n_extra;
+            link.moves_out[kPW + 1 + lane] = row_base + my_pos;
+            link.moves_out[2 * kPW + 1 + lane] = row_base + my_src;
         }
     } else {
         int pos[RPT];
@@ -900,20 +1062,21 @@ __global__ void __launch_bounds__(kPNa, 1)
 
 template <int RPT, bool MULTI>
 int32_t launch_panel32(Ctx* ctx, cudaStream_t st, int C, double* P, int64_t ld, int m, int w, int row_base,
-                       int col_base, int32_t* ipiv) {
+                       int col_base, int32_t* ipiv, const PanelLink& link) {
     auto kern = panel_kernel<RPT, MULTI>;
     const int R = (int)ceil_div(m, C);
-    constexpr size_t rcv = MULTI ? sizeof(PCand) * kPSlots * kPNw * kPMaxC : 0;
-    const size_t smem = (size_t)kPW * R * sizeof(double) + rcv;
+    constexpr size_t staged = (kPW * kPLRows + kPW * kPLtPitch) * sizeof(double);
+    constexpr size_t extra = MULTI ? sizeof(PCand) * kPSlots * kPNw * kPMaxC : staged;
+    const size_t smem = (size_t)kPW * R * sizeof(double) + (MULTI || link.moves_in ? extra : 0);
     std::atomic<int>& attr = device_flag((const void*)kern, 0, ctx->device);
     if (!attr.load()) {
         B2M_CU(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         B2M_CU(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(kPW * kPNt * RPT * sizeof(double) + rcv)));
+                                         (int)(kPW * kPNt * RPT * sizeof(double) + extra)));
         attr.store(1);
     }
     return launch_cluster(ctx, st, kern, C, kPNa, smem, m, w, sizeof(double), P, ld, m, w, R, row_base, col_base,
-                          ipiv, ctx->d_status);
+                          ipiv, ctx->d_status, link);
 }
 
 }  // namespace
@@ -927,7 +1090,7 @@ int panel_max_rows(bool fp64, int w) {
 
 template <typename T>
 int32_t launch_panel(Ctx* ctx, cudaStream_t st, T* P, int64_t ld, int m, int w, int row_base, int col_base,
-                     int32_t* ipiv) {
+                     int32_t* ipiv, const PanelLink& link) {
     if (w < 1 || w > 32 || m < w) return fail(ctx, B2M_ERR_DIM, "panel %d x %d", m, w);
     if constexpr (sizeof(T) == 8) {
         // Rows per thread (measured, 32 columns): up to 512 rows one CTA, 22.5 us at 256 rows with two
@@ -935,14 +1098,18 @@ int32_t launch_panel(Ctx* ctx, cudaStream_t st, T* P, int64_t ld, int m, int w, 
         // thread while 8 CTAs hold the panel (31.7 us at 1024 and 2048 rows; four: 37.8), then four,
         // which needs half the CTAs (38.0 us at 4096 rows; 38.9 on 16 CTAs).
         if (m <= kPMaxC * kPNt * 4 && aligned16(P) && ld % 2 == 0) {
-            if (m <= 2 * kPNt) return launch_panel32<2, false>(ctx, st, 1, P, ld, m, w, row_base, col_base, ipiv);
-            if (m <= 4 * kPNt) return launch_panel32<4, false>(ctx, st, 1, P, ld, m, w, row_base, col_base, ipiv);
+            if (m <= 2 * kPNt)
+                return launch_panel32<2, false>(ctx, st, 1, P, ld, m, w, row_base, col_base, ipiv, link);
+            if (m <= 4 * kPNt)
+                return launch_panel32<4, false>(ctx, st, 1, P, ld, m, w, row_base, col_base, ipiv, link);
             if (m <= 8 * 2 * kPNt)
                 return launch_panel32<2, true>(ctx, st, (int)ceil_div(m, 2 * kPNt), P, ld, m, w, row_base, col_base,
-                                               ipiv);
+                                               ipiv, link);
             return launch_panel32<4, true>(ctx, st, (int)ceil_div(m, 4 * kPNt), P, ld, m, w, row_base, col_base,
-                                           ipiv);
+                                           ipiv, link);
         }
+        if (link.moves_in || link.moves_out)
+            return fail(ctx, B2M_ERR_UNSUPPORTED, "a linked FP64 panel has at most %d rows", kPMaxC * kPNt * 4);
         if (w > 16) return fail(ctx, B2M_ERR_UNSUPPORTED, "FP64 panel of %d rows needs width <= 16", m);
         if (m > panel_max_rows(true, 16)) {  // very tall: 8 columns, 8 rows per thread
             const int C = (int)ceil_div(m, kPT * 8);
@@ -959,6 +1126,7 @@ int32_t launch_panel(Ctx* ctx, cudaStream_t st, T* P, int64_t ld, int m, int w, 
     }
 }
 
-template int32_t launch_panel<double>(Ctx*, cudaStream_t, double*, int64_t, int, int, int, int, int32_t*);
+template int32_t launch_panel<double>(Ctx*, cudaStream_t, double*, int64_t, int, int, int, int, int32_t*,
+                                      const PanelLink&);
 
 }  // namespace b2m
