@@ -6,20 +6,22 @@
 // magnitude <= 10/MaxDouble reporting the system singular (:246-268), forward substitution with the
 // unit-lower factor and back substitution dividing by U's diagonal (:315-385).
 //
-// Scheduling: the host sorts the systems largest first; resident CTAs pull them from an atomic work
-// queue (longest-processing-time first, no tail of big systems).  Systems of order > small_n take
-// a whole CTA; smaller ones are handed out in batches, one per group of G warps, each group with its
-// own named barrier.  The panel width of both size buckets and G are chosen by the autotuner at the
-// bottom of this file, which times the candidate shapes on the caller's batch.
+// The host sorts the systems largest first; resident CTAs pull them from an atomic work queue
+// (longest-processing-time first, no tail of big systems).
 //
-// Per system: A is copied into the CTA's private scratch slice (<= 256 x 256, L2 resident), where
-// a blocked right-looking LU runs with the current panel and the block row of U in shared memory.
-// Rows are never moved: a permutation maps factor rows to storage rows, so a pivot interchange swaps
-// two integers (the factors and the reference's interchange order are the same as with physical
-// swaps).  The solve is blocked by 32 rows: one warp per right-hand side substitutes a diagonal
-// block with shuffles, then the group folds it into the remaining rows.
+// Mode 0 (FP64): see batch_lu_kernel.
 //
-// Mode 1 factors in FP32 and refines in FP64: r = b - A x from the caller's FP64 A, d from the FP32
+// Mode 1: systems of order > small_n take a whole CTA; smaller ones are handed out in batches, one per
+// group of G warps, each group with its own named barrier.  The panel width of both size buckets and G
+// are chosen by the autotuner at the bottom of this file, which times the candidate shapes on the
+// caller's batch.  Per system a blocked right-looking LU runs on the CTA's private scratch slice
+// (<= 256 x 256, L2 resident) with the current panel and the block row of U in shared memory.  Rows are
+// never moved: a permutation maps factor rows to storage rows, so a pivot interchange swaps two integers
+// (the factors and the reference's interchange order are the same as with physical swaps).  The solve is
+// blocked by 32 rows: one warp per right-hand side substitutes a diagonal block with shuffles, then the
+// group folds it into the remaining rows.
+//
+// It factors in FP32 and refines in FP64: r = b - A x from the caller's FP64 A, d from the FP32
 // factors, x += d, until the normwise backward error max_q ||r_q|| / (||A|| ||x_q|| + ||b_q||) is
 // <= n 2^-53; a stall or an FP32 pivot <= 10/FLT_MAX refactors that system in FP64.
 #include <algorithm>
@@ -52,7 +54,8 @@ struct BatchArgs {
     const double* A;
     const double* B;
     double* X;
-    double* scratch;  // kBMaxN^2 doubles per CTA
+    double* scratch;  // the CTAs' factors
+    int64_t scratch_cta;  // doubles per CTA (mode 0)
     const int32_t* order;
     int32_t* counter;
     int32_t* info;
@@ -527,9 +530,8 @@ __device__ int solve_mixed(const Grp& g, const Slice& s, const BatchArgs& a, int
     return -1;
 }
 
-// MODE 0 plain FP64, 1 FP32 factor + FP64 refinement.  At most 128 registers a thread, so that
+// FP32 factor + FP64 refinement (mode 1).  At most 128 registers a thread, so that
 // two CTAs share an SM whenever the tile shape's shared memory allows it.
-template <int MODE>
 __global__ void __launch_bounds__(kBThreads, 2) batch_solve_kernel(BatchArgs a) {
     extern __shared__ __align__(16) double bsm[];
     __shared__ int s_sys[8];
@@ -561,16 +563,623 @@ __global__ void __launch_bounds__(kBThreads, 2) batch_solve_kernel(BatchArgs a) 
             const Grp g{t - gi * 32 * gw, 32 * gw, 2 + gi};
             const Slice s = carve(bsm + (size_t)gi * slice_doubles(nmax, pw), nmax, pw);
             double* Wg = W + (size_t)gi * nmax * nmax;
-            int st, iters = 0;
-            if (MODE == 1) {
-                iters = solve_mixed(g, s, a, msys, Wg);
-                st = iters < 0 ? solve_plain(g, s, a, msys, Wg) : 0;
-            } else {
-                st = solve_plain(g, s, a, msys, Wg);
-            }
+            const int iters = solve_mixed(g, s, a, msys, Wg);
+            const int st = iters < 0 ? solve_plain(g, s, a, msys, Wg) : 0;
             if (g.tid == 0) {
                 a.info[msys] = st;
                 if (a.iters) a.iters[msys] = iters;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// FP64 systems (mode 0): one launch of persistent CTAs of four warps, three to an SM.  A CTA takes one
+// system of order > 128 on all four warps, two of order 65 .. 128 on two warps each, or four smaller
+// ones on a warp each.  What bounds a system is the chain of its columns (pivot search, reciprocal,
+// update of the next column), so the chain is kept short and several systems share an SM to fill it:
+//   * leaves of 32 (16 for two warps or one) columns, their rows in shared memory and, eight columns
+//     at a time, in registers that shift left by one per column (a compact loop; see panel.cu, whose
+//     elimination this is for one CTA): one barrier a column;
+//   * rows never move: a thread carries its rows' positions, a permutation maps positions to rows;
+//   * the right-hand sides are extra columns, so L is never stored and needs no forward sweep;
+//   * U12 and the trailing update with it run on the FP64 tensor cores, a strip of columns per warp
+//     from registers (lu_strip);
+//   * the back substitution multiplies by the diagonal's reciprocal and corrects by the exact residual
+//     (as accurate as the division, whose 144 cycles would be on its chain 256 times), one warp per
+//     block with four lanes a right-hand side, and folds blocks on the tensor cores.
+// The matrix is worked on in the CTA's scratch (L2); the first leaf and update read A itself.
+// Measured on a B200: 20,000 systems of order 8 .. 256, k 1 .. 4: 23.0 ms before (panel and update of a
+// system on 8 warps, the panel in shared memory) and 8.8 ms (6.5 TFLOP/s) now; one system alone of order
+// 100 94 us, 256 326 us.
+// ------------------------------------------------------------------------------------------
+constexpr int kLuThreads = 128;
+constexpr int kLuCtas = 3;           // CTAs per SM the registers and the shared memory allow
+constexpr int kBk = 8;               // columns per register block
+
+struct __align__(16) LuCand {
+    double rinv;      // 1 / row[0]
+    int pos, lrow;    // position below the leaf's top, row in S
+    double row[kBk];  // the row's block columns, from the current one on
+};
+
+// shared memory of one group
+template <int NW, int W> struct LuSlice {
+    static constexpr int kRows = NW * 64;
+    double S[kRows * W];         // the leaf's rows, 16-byte pairs swizzled by row
+    double u[W * W];             // U11; then L11^T
+    double l8[kBk * kBk];        // a block's L
+    LuCand cand[2][NW];
+    __align__(16) uint32_t key[2][4];  // leading words of the candidates
+    int pl[W];                   // pivot rows in S
+    uint16_t perm[kRows];        // position -> row of the matrix
+    uint16_t lrow[kRows];        // live position -> row in S
+};
+
+template <int NW> __device__ __forceinline__ void lu_sync(int bar) {
+    if constexpr (NW == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "n"(NW * 32) : "memory");
+}
+__device__ __forceinline__ uint32_t lu_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
+
+// lane of the largest a >= 0 (the lowest pos among equals), compared exactly
+__device__ __noinline__ int lu_winner(double a, int pos) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+    const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
+    const uint32_t mhi = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+    const bool top = hi == mhi && lo == mlo;
+    const uint32_t mp = __reduce_min_sync(0xffffffffu, top ? (uint32_t)pos : 0xffffffffu);
+    return __ffs(__ballot_sync(0xffffffffu, top && (uint32_t)pos == mp)) - 1;
+}
+
+// Leaf of w <= W columns over m rows (loaded in s.S, zero past column w): eliminates with partial
+// pivoting.  pos[r] of row t + r * NW * 32 (its position on entry): its position afterwards, or
+// -1 - j for the pivot of column j.  Multipliers are left in S, U11 in s.u.  False: singular.
+template <int NW, int W>
+__device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w, int m, int (&pos)[2]) {
+    constexpr int NT = NW * 32, RPT = 2;
+    const int lane = t & 31, warp = t >> 5;
+    double* S = s.S;
+    auto sx = [](int row, int c) { return row * W + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
+    double act[RPT][kBk];
+#pragma unroll
+    for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int i = 0; i < kBk; i += 2) {
+            const double2 x = pos[r] >= 0 ? *reinterpret_cast<const double2*>(S + sx(t + r * NT, i))
+                                          : make_double2(0.0, 0.0);
+            act[r][i] = x.x; act[r][i + 1] = x.y;
+        }
+    auto publish = [&](const int col) {
+        uint32_t h[RPT];
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) h[r] = pos[r] >= 0 ? lu_hi(act[r][0]) : 0u;
+        const uint32_t mh = max(h[0], h[1]);
+        const bool second = h[1] > h[0];
+        double cr[kBk];
+#pragma unroll
+        for (int i = 0; i < kBk; ++i) cr[i] = second ? act[1][i] : act[0][i];
+        int cp = second ? pos[1] : pos[0], cl = second ? t + NT : t;
+        cr[0] = mh != 0 ? cr[0] : 0.0;
+        double rarg;  // opaque: a lane without a candidate must not divide by its zero (slow path)
+        asm("{ .reg .pred p; setp.ne.u32 p, %2, 0; selp.f64 %0, %1, 0d3FF0000000000000, p; }"
+            : "=d"(rarg)
+            : "d"(cr[0]), "r"(mh));
+        double rinv = 1.0 / rarg;
+        const uint32_t M = __reduce_max_sync(0xffffffffu, mh);
+        const uint32_t b1 = __ballot_sync(0xffffffffu, mh == M);
+        const uint32_t b2 = __ballot_sync(0xffffffffu, mh == M && h[0] == h[1]);
+        int wl = __ffs(b1) - 1;
+        if (M != 0 && ((b1 & (b1 - 1)) || b2 || M >= 0x7ff00000u)) {
+            double ba = 0.0;
+            cp = 0x7fffffff;
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) {
+                const double a = fabs(act[r][0]);
+                if (pos[r] >= 0 && a > 0.0 && (a > ba || (a == ba && pos[r] < cp))) {
+                    ba = a;
+                    cp = pos[r];
+                    cl = t + r * NT;
+#pragma unroll
+                    for (int i = 0; i < kBk; ++i) cr[i] = act[r][i];
+                }
+            }
+            if (!(ba > 0.0)) cr[0] = 0.0;
+            rinv = 1.0 / (ba > 0.0 ? cr[0] : 1.0);
+            wl = lu_winner(ba, cp);
+        }
+        if (lane == wl) {
+            LuCand& c = s.cand[col & 1][warp];
+#pragma unroll
+            for (int i = 0; i < kBk; i += 2)
+                *reinterpret_cast<double2*>(&c.row[i]) = make_double2(cr[i], cr[i + 1]);
+            c.rinv = rinv;
+            *reinterpret_cast<int2*>(&c.pos) = make_int2(M != 0 ? cp : 0x7fffffff, cl);
+            s.key[col & 1][warp] = lu_hi(cr[0]);
+        }
+    };
+    publish(0);
+    for (int jb = 0; jb < w; jb += kBk) {
+        const int bw = min(kBk, w - jb);
+#pragma unroll 1
+        for (int q = 0; q < bw; ++q) {
+            const int j = jb + q;
+            lu_sync<NW>(bar);
+            int win = 0;
+            if constexpr (NW > 1) {
+                const uint4 kv = *reinterpret_cast<const uint4*>(&s.key[j & 1][0]);
+                const uint32_t k[4] = {kv.x, kv.y, kv.z, kv.w};
+                uint32_t M = k[0];
+                int n = 0;
+#pragma unroll
+                for (int e = 1; e < NW; ++e) M = max(M, k[e]);
+#pragma unroll
+                for (int e = NW - 1; e >= 0; --e) {
+                    win = k[e] == M ? e : win;
+                    n += k[e] == M ? 1 : 0;
+                }
+                if (n > 1) {
+                    win = lu_winner(lane < NW ? fabs(s.cand[j & 1][lane].row[0]) : 0.0,
+                                    lane < NW ? s.cand[j & 1][lane].pos : 0x7fffffff);
+                    if (win >= NW) win = 0;
+                }
+            }
+            const LuCand& b = s.cand[j & 1][win];
+            double u[kBk];
+#pragma unroll
+            for (int i = 0; i < kBk; i += 2) {
+                const double2 x = *reinterpret_cast<const double2*>(&b.row[i]);
+                u[i] = x.x; u[i + 1] = x.y;
+            }
+            const double rinv = b.rinv;
+            const int2 pl = *reinterpret_cast<const int2*>(&b.pos);
+            if (!(fabs(u[0]) > sing_thresh<double>())) return false;  // uniform: every warp read the same
+            if (warp == NW - 1) {  // the pivot row's part of U inside its block
+                if (lane < kBk && q + lane < kBk && j + lane < W) s.u[j * W + j + lane] = b.row[lane];
+                if (lane == 0) s.pl[j] = pl.y;
+            }
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) {
+                const int rl = t + r * NT;
+                if (rl == pl.y) pos[r] = -1 - j;
+                else if (pos[r] == j) pos[r] = pl.x;
+                const double l = act[r][0] * rinv + 0.0;
+                if (pos[r] >= 0) S[sx(rl, j)] = l;
+#pragma unroll
+                for (int i = 1; i < kBk; ++i) act[r][i - 1] = fma(-l, u[i], act[r][i]);
+                act[r][kBk - 1] = 0.0;
+            }
+            if (q + 1 < bw) publish(j + 1);
+        }
+        const int c1 = jb + kBk;
+        if (c1 >= w) break;
+        // block end: the pivot rows right of the block, solved with the block's L
+        lu_sync<NW>(bar);
+        for (int e = t; e < kBk * (W / 2); e += NT) {
+            const int q = e / (W / 2), c = 2 * (e - q * (W / 2));
+            const double2 x = *reinterpret_cast<const double2*>(S + sx(s.pl[jb + q], c));
+            if (c >= c1) *reinterpret_cast<double2*>(&s.u[(jb + q) * W + c]) = x;
+            else if (c >= jb) *reinterpret_cast<double2*>(&s.l8[q * kBk + c - jb]) = x;
+        }
+        lu_sync<NW>(bar);
+        if (warp == 0 && c1 + lane < W) {
+            const int c = c1 + lane;
+            double x[kBk];
+#pragma unroll
+            for (int q = 0; q < kBk; ++q) x[q] = s.u[(jb + q) * W + c];
+#pragma unroll
+            for (int q0 = 0; q0 < kBk - 1; ++q0)
+#pragma unroll
+                for (int q1 = q0 + 1; q1 < kBk; ++q1) x[q1] = fma(-s.l8[q1 * kBk + q0], x[q0], x[q1]);
+#pragma unroll
+            for (int q = 1; q < kBk; ++q) s.u[(jb + q) * W + c] = x[q];
+        }
+        double l[RPT][kBk];
+#pragma unroll
+        for (int r = 0; r < RPT; ++r)
+#pragma unroll
+            for (int q = 0; q < kBk; q += 2) {
+                double2 x = make_double2(0.0, 0.0), y = x;
+                if (pos[r] >= 0) {
+                    x = *reinterpret_cast<const double2*>(S + sx(t + r * NT, jb + q));
+                    y = *reinterpret_cast<const double2*>(S + sx(t + r * NT, c1 + q));
+                }
+                l[r][q] = x.x; l[r][q + 1] = x.y;
+                act[r][q] = y.x; act[r][q + 1] = y.y;
+            }
+        lu_sync<NW>(bar);
+#pragma unroll
+        for (int i = 0; i < kBk; i += 2)
+#pragma unroll
+            for (int q = 0; q < kBk; ++q) {
+                const double2 uu = *reinterpret_cast<const double2*>(&s.u[(jb + q) * W + c1 + i]);
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) {
+                    act[r][i] = fma(-l[r][q], uu.x, act[r][i]);
+                    act[r][i + 1] = fma(-l[r][q], uu.y, act[r][i + 1]);
+                }
+            }
+        publish(c1);
+#pragma unroll 1
+        for (int c = c1 + kBk; c < w; c += 2) {
+            double2 x[RPT];
+#pragma unroll
+            for (int r = 0; r < RPT; ++r)
+                x[r] = pos[r] >= 0 ? *reinterpret_cast<const double2*>(S + sx(t + r * NT, c)) : make_double2(0.0, 0.0);
+#pragma unroll
+            for (int q = 0; q < kBk; ++q) {
+                const double2 uu = *reinterpret_cast<const double2*>(&s.u[(jb + q) * W + c]);
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) {
+                    x[r].x = fma(-l[r][q], uu.x, x[r].x);
+                    x[r].y = fma(-l[r][q], uu.y, x[r].y);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RPT; ++r)
+                if (pos[r] >= 0) *reinterpret_cast<double2*>(S + sx(t + r * NT, c)) = x[r];
+        }
+    }
+    return true;
+}
+
+__device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+                 : "d"(a0), "d"(a1), "d"(b));
+}
+
+// A strip of 16 columns from q0 on, right of the leaf [c0, c0 + w): U12 = L11^-1 A12 in registers,
+// then the strip's part of the trailing update with it, on the FP64 tensor cores (m16n8k4).
+//
+// Lane (g, t) = (lane / 4, lane % 4) holds of every 8 rows of A12 rows 2 t and 2 t + 1, columns g and
+// g + 8 of each 16: the accumulator layout of X^T (16 columns x 8 rows), which is also the operand
+// layout of X^T for the blocks below and of U12 for the trailing update when the k index of step s
+// (0, 1) counts rows 2 t + s.  So neither shared memory nor shuffles lie between the solve and the
+// updates; only the 8 x 8 triangles go by substitution, with a shuffle per row.  (A thread per column
+// read each multiplier by a broadcast, which costs the SM's shared memory 2 cycles per warp: 10,600
+// cycles a leaf of order 256.)
+template <int NW, int W, bool kFirst>
+__device__ __forceinline__ void lu_strip(LuSlice<NW, W>& s, int lane, const double* A, const double* B, int n, int kk,
+                                         int ld, double* V, int c0, int w, int q0) {
+    const int g = lane >> 2, t = lane & 3, nt = n + kk, cb = c0 + w, mr = n - cb;
+    auto sx = [](int row, int c) { return row * W + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
+    // Element (row, col) as this step finds it: A and B before the first update (kFirst).  Columns past
+    // the last one read it again, so that no load hides behind a branch; they are not stored.
+    auto at = [&](int row, int col) {
+        const int c = min(col, nt - 1);
+        if constexpr (kFirst) return c < n ? A[row * n + c] : B[row * kk + c - n];
+        else return V[row * ld + c];
+    };
+    double x[W / 8][4];
+#pragma unroll
+    for (int b = 0; b < W / 8; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int row = s.perm[c0 + min(8 * b + 2 * t + e, w - 1)];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) x[b][2 * h + e] = at(row, q0 + 8 * h + g);
+        }
+    // Rows past w (the last leaf of a matrix) hold copies of its last row: nothing depends on them and
+    // they are not stored.
+#pragma unroll
+    for (int b = 0; b < W / 8; ++b) {
+        const int pa = s.pl[min(8 * b + 2 * t, w - 1)], pb = s.pl[min(8 * b + 2 * t + 1, w - 1)];
+        double2 la[4], lb[4];  // this lane's two rows of the triangle
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            la[r] = *reinterpret_cast<const double2*>(s.S + sx(pa, 8 * b + 2 * r));
+            lb[r] = *reinterpret_cast<const double2*>(s.S + sx(pb, 8 * b + 2 * r));
+        }
+#pragma unroll
+        for (int r = 0; r < 7; ++r) {
+            const double ma = r & 1 ? la[r / 2].y : la[r / 2].x, mb = r & 1 ? lb[r / 2].y : lb[r / 2].x;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const double v = __shfl_sync(0xffffffffu, x[b][2 * h + (r & 1)], (lane & ~3) + r / 2);
+                if (2 * t > r) x[b][2 * h] = fma(-ma, v, x[b][2 * h]);
+                if (2 * t + 1 > r) x[b][2 * h + 1] = fma(-mb, v, x[b][2 * h + 1]);
+            }
+        }
+#pragma unroll
+        for (int b2 = b + 1; b2 < W / 8; ++b2) {
+            const double2 l = *reinterpret_cast<const double2*>(s.S + sx(s.pl[min(8 * b2 + g, w - 1)], 8 * b + 2 * t));
+            dmma(x[b2], x[b][0], x[b][2], -l.x);
+            dmma(x[b2], x[b][1], x[b][3], -l.y);
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < W / 8; ++b)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int j = 8 * b + 2 * t + e;
+            double* dst = V + s.perm[c0 + min(j, w - 1)] * ld + q0 + g;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (j < w && q0 + g + 8 * h < nt) dst[8 * h] = x[b][2 * h + e];
+                x[b][2 * h + e] = -x[b][2 * h + e];
+            }
+        }
+    if (mr <= 0) return;
+    // Rows below (w = W): 16 x 8 tiles, c = rows g, g + 8, columns 2 t, 2 t + 1; the next tile's old
+    // values are in flight under this one's products.  Pairs of columns are aligned in V, whose rows
+    // have a spare element where their length is odd; tiles past the last row repeat it.
+    double old[2][4];
+    int ro[2];
+    auto fetch = [&](int r0, int (&rows)[2]) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) rows[e] = s.perm[cb + min(r0 + g + 8 * e, mr - 1)];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int c = q0 + 8 * h + 2 * t;
+                if constexpr (kFirst) {
+                    old[h][2 * e] = at(rows[e], c);
+                    old[h][2 * e + 1] = at(rows[e], c + 1);
+                } else {
+                    const double2 v = *reinterpret_cast<const double2*>(V + rows[e] * ld + min(c, ld - 2));
+                    old[h][2 * e] = v.x;
+                    old[h][2 * e + 1] = v.y;
+                }
+            }
+    };
+    fetch(0, ro);
+#pragma unroll 1
+    for (int r0 = 0; r0 < mr; r0 += 16) {
+        double acc[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[h][e] = old[h][e];
+        const int la = s.lrow[w + min(r0 + g, mr - 1)], lb = s.lrow[w + min(r0 + g + 8, mr - 1)];
+        int rn[2] = {ro[0], ro[1]};
+        if (r0 + 16 < mr) fetch(r0 + 16, rn);
+#pragma unroll
+        for (int b = 0; b < W / 8; ++b) {
+            const double2 a0 = *reinterpret_cast<const double2*>(s.S + sx(la, 8 * b + 2 * t));
+            const double2 a1 = *reinterpret_cast<const double2*>(s.S + sx(lb, 8 * b + 2 * t));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                dmma(acc[h], a0.x, a1.x, x[b][2 * h]);
+                dmma(acc[h], a0.y, a1.y, x[b][2 * h + 1]);
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            double* dst = V + ro[e] * ld + q0 + 2 * t;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (r0 + g + 8 * e < mr && q0 + 8 * h + 2 * t < nt)
+                    *reinterpret_cast<double2*>(dst + 8 * h) = make_double2(acc[h][2 * e], acc[h][2 * e + 1]);
+        }
+        ro[0] = rn[0];
+        ro[1] = rn[1];
+    }
+}
+
+// One system on a group of NW warps; V is its scratch (row stride ld, 16-byte aligned rows).  0, or 1
+// when singular (uniform over the group).
+template <int NW, int W>
+__device__ __forceinline__ int lu_system(LuSlice<NW, W>& s, int t, int bar, const double* A, const double* B, double* X,
+                                         int n, int kk, double* V) {
+    constexpr int NT = NW * 32;
+    const int lane = t & 31, warp = t >> 5, ld = (n + kk + 1) & ~1, nt = n + kk;
+    auto sx = [](int row, int c) { return row * W + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
+    for (int i = t; i < n; i += NT) s.perm[i] = (uint16_t)i;
+    lu_sync<NW>(bar);
+    for (int c0 = 0; c0 < n; c0 += W) {
+        const bool first = c0 == 0;
+        const int w = min(W, n - c0), m = n - c0, cb = c0 + w;
+        if (first) {
+#pragma unroll 4
+            for (int e = t; e < m * W; e += NT) {
+                const int rl = e / W, c = e % W;
+                cp_async8(s.S + sx(rl, c), c < w ? A + (int64_t)rl * n + c : A, c < w ? 8 : 0);
+            }
+        } else {
+#pragma unroll 4
+            for (int e = t; e < m * (W / 2); e += NT) {
+                const int rl = e / (W / 2), c = 2 * (e % (W / 2));
+                cp_async16(s.S + sx(rl, c), c < w ? V + s.perm[c0 + rl] * ld + c0 + c : V,
+                           c + 1 < w ? 16 : (c < w ? 8 : 0));
+            }
+        }
+        cp_async_commit();
+        int pos[2], row[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int rl = t + r * NT;
+            pos[r] = rl < m ? rl : -1 - W;
+            row[r] = rl < m ? s.perm[c0 + rl] : 0;
+        }
+        cp_async_wait<0>();
+        lu_sync<NW>(bar);
+        if (!lu_leaf<NW, W>(s, t, bar, w, m, pos)) return 1;
+        lu_sync<NW>(bar);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int rl = t + r * NT;
+            if (rl < m) s.perm[c0 + (pos[r] < 0 ? -1 - pos[r] : pos[r])] = (uint16_t)row[r];
+            if (rl < m && pos[r] >= 0) s.lrow[pos[r]] = (uint16_t)rl;
+        }
+        lu_sync<NW>(bar);
+        for (int e0 = t; e0 < W * W; e0 += 4 * NT) {  // U11
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int e = e0 + i * NT, j = e / W, c = e % W;
+                if (j < w && c >= j && c < w) V[s.perm[c0 + j] * ld + c0 + c] = s.u[e];
+            }
+        }
+        // the columns to the right, 16 a warp (strips of 32 took 10.5 ms instead of 8.8: more registers
+        // than three CTAs an SM allow, and idle warps on the last columns)
+        auto strips = [&](auto first) {
+            constexpr bool kFirst = decltype(first)::value;
+            for (int q0 = cb + 16 * warp; q0 < nt; q0 += 16 * NW)
+                lu_strip<NW, W, kFirst>(s, lane, A, B, n, kk, ld, V, c0, w, q0);
+        };
+        if (first) strips(std::true_type{});
+        else strips(std::false_type{});
+        lu_sync<NW>(bar);
+    }
+    // ---- back substitution: y (n x 8, zero past kk) in S's place, a block of U in u
+    double* y = s.S;
+    for (int e = t; e < n * kBMaxK; e += NT) {
+        const int j = e / kBMaxK, q = e % kBMaxK;
+        y[e] = q < kk ? V[s.perm[j] * ld + n + q] : 0.0;
+    }
+    for (int b0 = (n - 1) / W * W; b0 >= 0; b0 -= W) {
+        const int bs = min(W, n - b0);
+        lu_sync<NW>(bar);
+        batched_copy<NT, 8, double>(t, W * W,  // the block's columns: u[c][r] = U(b0 + r, b0 + c), identity past bs
+            [&](int e) {
+                const int r = e / W, c = e % W;
+                return (r <= c && c < bs) ? V[s.perm[b0 + r] * ld + b0 + c] : (r == c ? 1.0 : 0.0);
+            },
+            [&](int e, double v) { s.u[e % W * W + e / W] = v; });
+        lu_sync<NW>(bar);
+        if (warp == 0) {
+            // lane = right-hand side + 8 * (row & 3); rows from the last one up, four a step.  x / d is
+            // the product with the reciprocal corrected by its exact residual; where a diagonal is far
+            // from 1 or a result is not finite, the block is solved again with divisions.
+            const int q = lane & 7, rg = lane >> 3;
+            double dv[W / 4], di[W / 4];
+            bool odd = false;
+#pragma unroll
+            for (int i = 0; i < W / 4; ++i) {
+                dv[i] = s.u[(4 * i + rg) * (W + 1)];
+                di[i] = 1.0 / dv[i];
+                odd = odd || lu_hi(dv[i]) - 0x01700000u >= 0x7d000000u;  // outside 2^-1000 .. 2^1000
+            }
+            double y0[W / 4];
+#pragma unroll
+            for (int i = 0; i < W / 4; ++i) y0[i] = 4 * i + rg < bs ? y[(b0 + 4 * i + rg) * kBMaxK + q] : 0.0;
+            auto solve = [&](auto divide) {
+                constexpr bool kDivide = decltype(divide)::value;
+                constexpr int kTop = W / 4 - 1;
+                double x[W / 4], d[W / 4], r[W / 4];
+#pragma unroll
+                for (int i = 0; i < W / 4; ++i) {
+                    x[i] = y0[i];
+                    d[i] = dv[i];
+                    r[i] = di[i];
+                }
+                bool finite = true;
+#pragma unroll 1
+                for (int i4 = kTop; i4 >= 0; --i4) {
+#pragma unroll
+                    for (int v = 3; v >= 0; --v) {
+                        const double z = x[kTop];
+                        double xq;
+                        if constexpr (kDivide) {
+                            xq = z / d[kTop];
+                        } else {
+                            xq = z * r[kTop];
+                            xq = fma(fma(-xq, d[kTop], z), r[kTop], xq);
+                        }
+                        const double xj = __shfl_sync(0xffffffffu, xq, q + 8 * v);
+                        if (rg == v) x[kTop] = xq;
+                        const double* uc = &s.u[(4 * i4 + v) * W + rg];
+                        if (rg < v) x[kTop] = fma(-uc[4 * i4], xj, x[kTop]);
+#pragma unroll
+                        for (int i = 1; i < W / 4; ++i)
+                            if (i4 - i >= 0) x[kTop - i] = fma(-uc[4 * (i4 - i)], xj, x[kTop - i]);
+                    }
+                    finite = finite && lu_hi(x[kTop]) < 0x7ff00000u;
+                    if (4 * i4 + rg < bs) y[(b0 + 4 * i4 + rg) * kBMaxK + q] = x[kTop];
+#pragma unroll
+                    for (int i = kTop; i > 0; --i) {
+                        x[i] = x[i - 1];
+                        d[i] = d[i - 1];
+                        r[i] = r[i - 1];
+                    }
+                }
+                return finite;
+            };
+            bool again = __any_sync(0xffffffffu, odd);
+            if (!again) again = !__all_sync(0xffffffffu, solve(std::false_type{}));
+            if (again) solve(std::true_type{});
+        }
+        lu_sync<NW>(bar);
+        // fold the block into the rows above (only full blocks of 4 k: bs < W only in the last one)
+        const int g = lane >> 2, tq = lane & 3;
+        for (int r0 = 16 * warp; r0 < b0; r0 += 16 * NW) {
+            const int ra = s.perm[r0 + g] * ld + b0, rb = s.perm[r0 + g + 8] * ld + b0;  // (b0 is a multiple of 16)
+            double a0[W / 4], a1[W / 4], acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < W / 4; ++k) {
+                const bool in = 4 * k + tq < bs;
+                a0[k] = in ? V[ra + 4 * k + tq] : 0.0;
+                a1[k] = in ? V[rb + 4 * k + tq] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < W / 4; ++k) {
+                const double b = 4 * k + tq < bs ? y[(b0 + 4 * k + tq) * kBMaxK + g] : 0.0;
+                asm volatile(
+                    "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+                    : "+d"(acc[0]), "+d"(acc[1]), "+d"(acc[2]), "+d"(acc[3])
+                    : "d"(a0[k]), "d"(a1[k]), "d"(b));
+            }
+            double2* ya = reinterpret_cast<double2*>(y + (r0 + g) * kBMaxK + 2 * tq);
+            double2* yb = reinterpret_cast<double2*>(y + (r0 + g + 8) * kBMaxK + 2 * tq);
+            *ya = make_double2(ya->x - acc[0], ya->y - acc[1]);
+            *yb = make_double2(yb->x - acc[2], yb->y - acc[3]);
+        }
+    }
+    lu_sync<NW>(bar);
+    for (int e = t; e < n * kk; e += NT) X[e] = y[e / kk * kBMaxK + e % kk];
+    lu_sync<NW>(bar);
+    return 0;
+}
+
+// scratch of one system with its right-hand sides; of a CTA in a batch whose largest order is nmax
+__host__ __device__ constexpr int64_t lu_mat(int n) { return (int64_t)n * ((n + kBMaxK + 1) & ~1); }
+int64_t lu_scratch(int nmax) { return std::max(nmax > 64 ? 2 * lu_mat(128) : 4 * lu_mat(64), lu_mat(nmax)); }
+
+union LuShared {
+    LuSlice<4, 32> one;
+    LuSlice<2, 16> two[2];
+    LuSlice<1, 16> four[4];
+};
+
+// As many CTAs as systems: the time of one counts, not how many an SM holds (four warps each against two or
+// one: order 100 95 / 115 us, 200 of order 60 60 / 68 us, 440 of order 100 131 / 134 us).
+bool lu_wide(int64_t count, int num_sms) { return count <= (int64_t)num_sms * kLuCtas; }
+
+// wide: every system runs on four warps (few systems, where the time of one counts)
+__global__ void __launch_bounds__(kLuThreads, kLuCtas) batch_lu_kernel(BatchArgs a, int wide) {
+    extern __shared__ __align__(16) unsigned char lu_dyn[];
+    LuShared& sh = *reinterpret_cast<LuShared*>(lu_dyn);
+    __shared__ int s_sys[4];
+    const int t = threadIdx.x;
+    double* V = a.scratch + (size_t)blockIdx.x * a.scratch_cta;
+    for (;;) {
+        if (t == 0) s_sys[0] = atomicAdd(a.counter, 1);
+        __syncthreads();
+        const int idx = s_sys[0];
+        if (idx >= a.count) return;
+        // the queue is sorted largest first: the systems that follow are no larger
+        const int n0 = a.n[a.order[idx]];
+        const int groups = wide || n0 > 128 ? 1 : (n0 > 64 ? 2 : 4);
+        if (t > 0 && t < groups) {
+            const int j = atomicAdd(a.counter, 1);
+            s_sys[t] = j < a.count ? j : -1;
+        }
+        __syncthreads();
+        const int gi = t / (kLuThreads / groups), myidx = s_sys[gi], gt = t - gi * (kLuThreads / groups);
+        if (myidx >= 0) {
+            const int sys = a.order[myidx], n = a.n[sys], kk = a.k[sys];
+            const double *A = a.A + a.a_off[sys], *B = a.B + a.b_off[sys];
+            double* X = a.X + a.b_off[sys];
+            int st;
+            if (groups == 1) st = lu_system<4, 32>(sh.one, gt, 1, A, B, X, n, kk, V);
+            else if (groups == 2) st = lu_system<2, 16>(sh.two[gi], gt, 1 + gi, A, B, X, n, kk, V + gi * lu_mat(128));
+            else st = lu_system<1, 16>(sh.four[gi], gt, 0, A, B, X, n, kk, V + gi * lu_mat(64));
+            if (gt == 0) {
+                a.info[sys] = st;
+                if (a.iters) a.iters[sys] = 0;
             }
         }
         __syncthreads();
@@ -651,7 +1260,7 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
 
     auto launch = [&](const BatchTune& tc, cudaStream_t q) -> int32_t {
         const size_t smem = batch_smem_bytes(tc.small_n, tc.group_warps, tc.pw_large, tc.pw_small, tc.big_warps);
-        void (*kern)(BatchArgs) = mode == 1 ? batch_solve_kernel<1> : batch_solve_kernel<0>;
+        void (*kern)(BatchArgs) = batch_solve_kernel;
         B2M_CU(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
         B2M_CU(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBThreads, smem));
@@ -676,11 +1285,36 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
         return B2M_OK;
     };
 
+    // mode 0 has one shape: nothing to tune (the table still lists the plan)
+    auto launch_lu = [&](cudaStream_t q) -> int32_t {
+        std::atomic<int>& attr = device_flag((const void*)batch_lu_kernel, 0, ctx->device);
+        if (!attr.load()) {
+            B2M_CU(ctx, cudaFuncSetAttribute(batch_lu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(LuShared)));
+            attr.store(1);
+        }
+        const int64_t grid = std::min<int64_t>(count, (int64_t)ctx->num_sms * kLuCtas);
+        void* pscr;
+        const int64_t per = lu_scratch(hn[order[0]]);
+        B2M_TRY(ws_get(ctx, kWsMatD, (size_t)(grid * per) * sizeof(double), &pscr));
+        BatchArgs b = a;
+        b.scratch = static_cast<double*>(pscr);
+        b.scratch_cta = per;
+        B2M_CU(ctx, cudaMemsetAsync(dctr, 0, sizeof(int32_t), q));
+        prof_begin(ctx, q, kClsSolve);
+        batch_lu_kernel<<<(unsigned)grid, kLuThreads, sizeof(LuShared), q>>>(b, lu_wide(count, ctx->num_sms) ? 1 : 0);
+        prof_end(ctx, q, kClsSolve, 0.0);
+        B2M_LAUNCHED(ctx);
+        return B2M_OK;
+    };
+
     // autotune once per plan (mode, sizes, layout): time each candidate shape on this batch
     BatchTune best;
     auto it = ctx->batch_tunes.find(sig);
     if (it != ctx->batch_tunes.end()) {
         best = it->second;
+    } else if (mode == 0) {
+        best = ctx->batch_tunes[sig] = BatchTune{64, 1, 32, 16, 8, 0.0f};
     } else {
         std::vector<BatchTune> cands;
         for (int GB : {8, 4})
@@ -713,7 +1347,7 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
     const GraphKey key{7 + mode * 10, A, B, X, info, count, (int64_t)sig,
                        best.big_warps * 1000000 + best.pw_large * 10000 + best.pw_small * 100 + best.group_warps,
                        (int64_t)reinterpret_cast<intptr_t>(iters)};
-    return run_graph(ctx, st, key, [&](cudaStream_t q) { return launch(best, q); });
+    return run_graph(ctx, st, key, [&](cudaStream_t q) { return mode == 0 ? launch_lu(q) : launch(best, q); });
 }
 
 }  // namespace b2m
