@@ -35,6 +35,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "panel.cuh"
 
 namespace b2m {
 namespace {
@@ -621,18 +622,6 @@ template <int NW> __device__ __forceinline__ void lu_sync(int bar) {
     if constexpr (NW == 1) __syncwarp();
     else asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "n"(NW * 32) : "memory");
 }
-__device__ __forceinline__ uint32_t lu_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
-
-// lane of the largest a >= 0 (the lowest pos among equals), compared exactly
-__device__ __noinline__ int lu_winner(double a, int pos) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-    const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
-    const uint32_t mhi = __reduce_max_sync(0xffffffffu, hi);
-    const uint32_t mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-    const bool top = hi == mhi && lo == mlo;
-    const uint32_t mp = __reduce_min_sync(0xffffffffu, top ? (uint32_t)pos : 0xffffffffu);
-    return __ffs(__ballot_sync(0xffffffffu, top && (uint32_t)pos == mp)) - 1;
-}
 
 // Leaf of w <= W columns over m rows (loaded in s.S, zero past column w): eliminates with partial
 // pivoting.  pos[r] of row t + r * NW * 32 (its position on entry): its position afterwards, or
@@ -655,7 +644,7 @@ __device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w
     auto publish = [&](const int col) {
         uint32_t h[RPT];
 #pragma unroll
-        for (int r = 0; r < RPT; ++r) h[r] = pos[r] >= 0 ? lu_hi(act[r][0]) : 0u;
+        for (int r = 0; r < RPT; ++r) h[r] = pos[r] >= 0 ? mag_hi(act[r][0]) : 0u;
         const uint32_t mh = max(h[0], h[1]);
         const bool second = h[1] > h[0];
         double cr[kBk];
@@ -672,7 +661,7 @@ __device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w
         const uint32_t b1 = __ballot_sync(0xffffffffu, mh == M);
         const uint32_t b2 = __ballot_sync(0xffffffffu, mh == M && h[0] == h[1]);
         int wl = __ffs(b1) - 1;
-        if (M != 0 && ((b1 & (b1 - 1)) || b2 || M >= 0x7ff00000u)) {
+        if (M != 0 && ((b1 & (b1 - 1)) || b2 || M >= kInfHi)) {
             double ba = 0.0;
             cp = 0x7fffffff;
 #pragma unroll
@@ -688,7 +677,7 @@ __device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w
             }
             if (!(ba > 0.0)) cr[0] = 0.0;
             rinv = 1.0 / (ba > 0.0 ? cr[0] : 1.0);
-            wl = lu_winner(ba, cp);
+            wl = warp_winner(ba, cp);
         }
         if (lane == wl) {
             LuCand& c = s.cand[col & 1][warp];
@@ -697,7 +686,7 @@ __device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w
                 *reinterpret_cast<double2*>(&c.row[i]) = make_double2(cr[i], cr[i + 1]);
             c.rinv = rinv;
             *reinterpret_cast<int2*>(&c.pos) = make_int2(M != 0 ? cp : 0x7fffffff, cl);
-            s.key[col & 1][warp] = lu_hi(cr[0]);
+            s.key[col & 1][warp] = mag_hi(cr[0]);
         }
     };
     publish(0);
@@ -721,7 +710,7 @@ __device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w
                     n += k[e] == M ? 1 : 0;
                 }
                 if (n > 1) {
-                    win = lu_winner(lane < NW ? fabs(s.cand[j & 1][lane].row[0]) : 0.0,
+                    win = warp_winner(lane < NW ? fabs(s.cand[j & 1][lane].row[0]) : 0.0,
                                     lane < NW ? s.cand[j & 1][lane].pos : 0x7fffffff);
                     if (win >= NW) win = 0;
                 }
@@ -1051,7 +1040,7 @@ __device__ __forceinline__ int lu_system(LuSlice<NW, W>& s, int t, int bar, cons
             for (int i = 0; i < W / 4; ++i) {
                 dv[i] = s.u[(4 * i + rg) * (W + 1)];
                 di[i] = 1.0 / dv[i];
-                odd = odd || lu_hi(dv[i]) - 0x01700000u >= 0x7d000000u;  // outside 2^-1000 .. 2^1000
+                odd = odd || mag_hi(dv[i]) - 0x01700000u >= 0x7d000000u;  // outside 2^-1000 .. 2^1000
             }
             double y0[W / 4];
 #pragma unroll
@@ -1087,7 +1076,7 @@ __device__ __forceinline__ int lu_system(LuSlice<NW, W>& s, int t, int bar, cons
                         for (int i = 1; i < W / 4; ++i)
                             if (i4 - i >= 0) x[kTop - i] = fma(-uc[4 * (i4 - i)], xj, x[kTop - i]);
                     }
-                    finite = finite && lu_hi(x[kTop]) < 0x7ff00000u;
+                    finite = finite && mag_hi(x[kTop]) < kInfHi;
                     if (4 * i4 + rg < bs) y[(b0 + 4 * i4 + rg) * kBMaxK + q] = x[kTop];
 #pragma unroll
                     for (int i = kTop; i > 0; --i) {

@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "panel.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -355,42 +356,6 @@ __global__ void __launch_bounds__(kPT, 1)
     cluster.sync();  // no CTA leaves while a push to it may still be in flight
 }
 
-// one cluster of C CTAs (a plain launch for C = 1) with the critical path's priority
-template <typename Kern, typename... Args>
-int32_t launch_cluster(Ctx* ctx, cudaStream_t st, Kern kern, int C, int threads, size_t smem, int m, int w,
-                       size_t elem, Args... args) {
-    // whether a cluster of C CTAs fits on this device: 1 yes, -1 no, 0 not asked yet
-    std::atomic<int>& sched = device_flag((const void*)kern, 1 + C, ctx->device);
-    cudaLaunchAttribute at[2];
-    // the panel is the factorisation's critical path: when a look-ahead trailing update runs beside
-    // it, its CTAs take free SMs ahead of the update's tiles
-    at[0].id = cudaLaunchAttributePriority;
-    at[0].val.priority = ctx->chain_priority;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = C;
-    at[1].val.clusterDim.y = 1;
-    at[1].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(C, 1, 1);
-    cfg.blockDim = dim3(threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = C > 1 ? 2 : 1;
-    if (C > 8 && sched.load() == 0) {
-        int clusters = 0;
-        B2M_CU(ctx, cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg));
-        sched.store(clusters > 0 ? 1 : -1);
-    }
-    if (C > 8 && sched.load() < 0)
-        return fail(ctx, B2M_ERR_UNSUPPORTED, "panel cluster of %d CTAs cannot be scheduled", C);
-    prof_begin(ctx, st, kClsPanel);
-    B2M_CU(ctx, cudaLaunchKernelEx(&cfg, kern, args...));
-    prof_end(ctx, st, kClsPanel, 2.0 * m * w * elem);  // bytes: the panel read and written once
-    B2M_LAUNCHED(ctx);
-    return B2M_OK;
-}
-
 template <typename T, int W, int RPT>
 int32_t launch_push(Ctx* ctx, cudaStream_t st, int C, int R, T* P, int64_t ld, int m, int w, int row_base,
                     int col_base, int32_t* ipiv) {
@@ -402,7 +367,7 @@ int32_t launch_push(Ctx* ctx, cudaStream_t st, int C, int R, T* P, int64_t ld, i
         B2M_CU(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmemMax));
         attr.store(1);
     }
-    return launch_cluster(ctx, st, kern, C, kPT, smem, m, w, sizeof(T), P, ld, m, w, R, row_base, col_base, ipiv,
+    return launch_cluster(ctx, st, kern, false, C, kPT, smem, m, w, sizeof(T), P, ld, m, w, R, row_base, col_base, ipiv,
                           ctx->d_status);
 }
 
@@ -442,20 +407,6 @@ constexpr int kPBk = 8;              // columns per block
 // Candidates are kept for 16 columns: a CTA may push column j + 16 only after every CTA has sent
 // column j + 15, and so has left the block of column j.
 constexpr int kPSlots = 2 * kPBk;
-constexpr unsigned kPInf = 0x7ff00000u;  // leading word of infinity
-
-__device__ __forceinline__ uint32_t mag_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
-
-// lane of the largest a >= 0 (the lowest pos among equals), compared exactly
-__device__ __noinline__ int warp_winner(double a, int pos) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-    const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
-    const uint32_t mhi = __reduce_max_sync(0xffffffffu, hi);
-    const uint32_t mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-    const bool top = hi == mhi && lo == mlo;
-    const uint32_t mp = __reduce_min_sync(0xffffffffu, top ? (uint32_t)pos : 0xffffffffu);
-    return __ffs(__ballot_sync(0xffffffffu, top && (uint32_t)pos == mp)) - 1;
-}
 
 // The previous leaf of the same outer panel (PanelLink::moves_in not null): the kernel first applies
 // its interchanges, its triangular solve and its rank-32 update to the leaf's own columns, which still
@@ -762,7 +713,7 @@ __global__ void __launch_bounds__(kPNa, 1)
             if (lane < kPBk && (j & (kPBk - 1)) + lane < kPBk && j + lane < kPW) s_u[j][j + lane] = v;
             if (lane == 0) {
                 if (rank == 0) ipiv[col_base + j] = row_base + b->pos;
-                s_pl[j] = b->lrow;
+                s_pl[j] = min((unsigned)b->lrow, (unsigned)R - 1u);  // (in range after a wait that ran out, too)
                 s_ps[j] = MULTI ? win / kPNw : 0;
             }
             if ((j & (kPBk - 1)) == kPBk - 1 && j + 1 < w) {
@@ -835,7 +786,7 @@ __global__ void __launch_bounds__(kPNa, 1)
             const uint32_t b1 = __ballot_sync(0xffffffffu, mh == M);
             const uint32_t b2 = __ballot_sync(0xffffffffu, mh == M && cnt > 1);
             int wl = __ffs(b1) - 1;
-            if (M != 0 && ((b1 & (b1 - 1)) || b2 || M >= kPInf)) {
+            if (M != 0 && ((b1 & (b1 - 1)) || b2 || M >= kInfHi)) {
                 double ba = 0.0;
                 cp = 0x7fffffff;
 #pragma unroll
@@ -1021,7 +972,7 @@ __global__ void __launch_bounds__(kPNa, 1)
             constexpr int BP = kPW / RS < 4 ? kPW / RS : 4, B = 8;
             const int c = 2 * (tid % LPR);
             auto put = [&](int row, double2 x) {
-                if (late) return;
+                if (late || row >= m) return;
                 double* dst = P + (int64_t)row * ld + c;
                 if (c + 1 < w) *reinterpret_cast<double2*>(dst) = x;
                 else if (c < w) *dst = x.x;
@@ -1075,7 +1026,7 @@ int32_t launch_panel32(Ctx* ctx, cudaStream_t st, int C, double* P, int64_t ld, 
                                          (int)(kPW * kPNt * RPT * sizeof(double) + extra)));
         attr.store(1);
     }
-    return launch_cluster(ctx, st, kern, C, kPNa, smem, m, w, sizeof(double), P, ld, m, w, R, row_base, col_base,
+    return launch_cluster(ctx, st, kern, !MULTI, C, kPNa, smem, m, w, sizeof(double), P, ld, m, w, R, row_base, col_base,
                           ipiv, ctx->d_status, link);
 }
 
