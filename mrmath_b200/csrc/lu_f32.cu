@@ -26,6 +26,7 @@
 // A pivot whose magnitude is <= 10/FLT_MAX at the root sets status[kInfo] (the driver then
 // falls back to the plain FP64 factorisation).
 #include <cfloat>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -70,141 +71,251 @@ __device__ __forceinline__ float rcp_nr(float x) {
 // t and t + 256 in registers) over w <= 32 columns.  Chooses w pivot rows (largest magnitude);
 // s_win[j] = row id of pivot j and s_loc[j] = its stack index (-1 if the stack ran out).
 //
-// One column per iteration of a runtime loop (a compact body: unrolled multi-column steps spill
-// out of the instruction cache).  Register indices stay compile-time because every row shifts
-// left by one as its column is eliminated (the update writes v[k - 1]), so the current column is
-// always v[0].  One barrier per column: before it, every warp's best lane publishes its candidate
-// row, the reciprocal of its pivot value (computed by every lane while the warp reduction runs,
-// so it is off the chain) and its stack slot (double-buffered by column parity), and folds its key
-// into a shared maximum (atomicMax on the magnitude's bit pattern with the warp in the low 3 bits,
-// so the lowest warp wins among magnitudes that agree to 2^-20); after it, every thread reads the
-// maximum and then the winning row directly, with no further reduction.  The maximum words rotate
-// through three slots: thread 0 clears the one of column j + 2 after the barrier of column j, when
-// every read of it (column j - 1) is done and before any write (column j + 2).  For the root (lm
-// given) the winner of column j is copied to s_u[j] (row j of U, from column j on) and every row's
-// multiplier of column j goes to lm[j][stack index] (global scratch), which gives the rows of L;
-// keeping them out of shared memory lets the CTA share an SM with a tensor-core GEMM.
+// What bounds it is the chain of one column: a warp reduction, a barrier, reading the winner, and the
+// instructions around them.  So
+//   * columns go in blocks of eight, and a column's step touches the block only: the columns to the
+//     right get the block's eight updates at once at its end, from the block's pivot rows (as their
+//     owners hold them, solved with the block's L11).  A step over all 32 columns read the whole pivot
+//     row in every warp, which costs the SM's shared memory a cycle per warp and element;
+//   * rows shift left by one as a column is eliminated, so the current column is always v[0]; the
+//     multipliers are kept in shared memory until the block's end;
+//   * one barrier a column: before it, every warp's best lane publishes its row's block part, its
+//     key (the magnitude with the warp in the low 3 bits, so that the lowest warp wins among magnitudes
+//     that agree to 2^-20) and the reciprocal of its pivot value (computed by every lane under the warp
+//     reduction), double-buffered by column parity; after it, every thread reads the eight keys and the
+//     winner.  Nothing diverges: the publishing lane's stores are predicated one by one (as a branch
+//     they took 190 cycles), a row's owner only notes its column, and rows past the leaf or the stack
+//     need no test (a zero column eliminates nothing, and without live rows nothing is chosen).
+// Every element sees the same products in the same order as column by column over all 32.  For the root
+// (lm given) the rows of U go to g.ur and every row's multiplier of column j to lm[j][stack index]
+// (global scratch), which gives the rows of L.
+// Measured on a B200 (cycles, 512 rows x 32 columns, the CTA alone): 32,500 -> 18,000; eight warps against
+// four with four rows a thread 19,000 to 18,700, a loop over the block's columns instead of their unrolled steps 21,400.
+constexpr int kTsWarps = kTsThreads / 32;
+// Shared memory that is asked for and not used: with it the few CTAs, which are the factorisation's critical
+// path, do not share their SMs with a tile of the trailing GEMM (an elimination beside one took 27,000 cycles);
+// one of the 148 SMs becomes free within about a microsecond.  Order 8192: 15.94 -> 15.73 ms.
+constexpr int kTsReserve = 120 * 1024;
+constexpr int kTsBk = 8;
+static_assert(kTsWarps == 8, "the warps' keys are read as two uint4, and have the warp in the low 3 bits");
+
 struct GeppSmem {
-    float4 cand[2][kTsThreads / 32][9];  // candidate rows by column parity and warp (column j first),
-                                         // then (reciprocal of the pivot, stack slot, -, -)
-    unsigned best[3];                    // packed maximum key of columns j, j + 1, j + 2 (mod 3)
-    float4 u[32][8];                     // root: pivot rows as chosen
+    float4 cand[2][kTsWarps][3];  // by column parity and warp: the row's block part (current column first),
+                                  // then (reciprocal of the pivot, stack slot, -, -)
+    uint4 key[2][2];              // the warps' magnitudes + 1 with 7 - warp in the low 3 bits (0: no live row)
+    float u[kTsBk][32 - kTsBk];   // the block's pivot rows right of the block
+    float ur[32][32];             // root: rows of U
 };
 
+// stores to shared memory where p, without a branch
+__device__ __forceinline__ void st_if(bool p, void* dst, float x, float y, float z, float w) {
+    asm volatile("{.reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.v4.f32 [%1], {%2, %3, %4, %5};}" ::"r"((unsigned)p),
+                 "r"(smem_u32(dst)), "f"(x), "f"(y), "f"(z), "f"(w)
+                 : "memory");
+}
+__device__ __forceinline__ void st_if(bool p, void* dst, float x, float y) {
+    asm volatile("{.reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.v2.f32 [%1], {%2, %3};}" ::"r"((unsigned)p),
+                 "r"(smem_u32(dst)), "f"(x), "f"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void st_if(bool p, void* dst, unsigned x) {
+    asm volatile("{.reg .pred p; setp.ne.u32 p, %0, 0; @p st.shared.u32 [%1], %2;}" ::"r"((unsigned)p),
+                 "r"(smem_u32(dst)), "r"(x)
+                 : "memory");
+}
+
+// mul: kTsBk x kTsRows floats of shared memory
 __device__ __forceinline__ void block_gepp(float (&v)[kTsRpt][32], const int (&rid)[kTsRpt], int w, int* s_win,
-                                           int* s_loc, GeppSmem& g, float* lm) {
-    static_assert(kTsThreads / 32 <= 8, "the warp index must fit the key's low 3 bits");
+                                           int* s_loc, GeppSmem& g, float* mul, float* lm) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    bool live[kTsRpt];
+    const unsigned below = (1u << lane) - 1u;
+    int pq[kTsRpt];  // the column whose pivot the row is; -1: live
 #pragma unroll
-    for (int r = 0; r < kTsRpt; ++r) live[r] = rid[r] >= 0;
+    for (int r = 0; r < kTsRpt; ++r) pq[r] = rid[r] >= 0 ? -1 : -2;
     if (t < 32) { s_win[t] = -1; s_loc[t] = -1; }
-    if (t < 3) g.best[t] = 0u;
     __syncthreads();
-    int b3 = 0;
 #pragma unroll 1
-    for (int j = 0; j < w; ++j) {
-        const int b = j & 1;
-        unsigned key = 0u;
-        int rbest = 0;
+    for (int jb = 0; jb < w; jb += kTsBk) {
 #pragma unroll
-        for (int r = 0; r < kTsRpt; ++r) {
-            const unsigned k = live[r] ? __float_as_uint(fabsf(v[r][0])) + 1u : 0u;
-            if (k > key) { key = k; rbest = r; }
-        }
-        float vsel = v[0][0];
+        for (int q = 0; q < kTsBk; ++q) {
+            const int b = q & 1;
+            unsigned key = pq[0] == -1 ? __float_as_uint(fabsf(v[0][0])) + 1u : 0u;
+            float c0 = v[0][0];
+            int rb = 0;
 #pragma unroll
-        for (int r = 1; r < kTsRpt; ++r) vsel = rbest == r ? v[r][0] : vsel;
-        const float rc = key > 1u ? rcp_nr(vsel) : 0.0f;  // a zero column eliminates nothing
-        const unsigned wk = __reduce_max_sync(0xffffffffu, key);
-        const unsigned bal = __ballot_sync(0xffffffffu, key == wk && key != 0u);
-        if (wk != 0u && lane == __ffs(bal) - 1) {
+            for (int r = 1; r < kTsRpt; ++r) {
+                const unsigned kr = pq[r] == -1 ? __float_as_uint(fabsf(v[r][0])) + 1u : 0u;
+                const bool is = kr > key;
+                key = is ? kr : key;
+                rb = is ? r : rb;
+                c0 = is ? v[r][0] : c0;
+            }
+            const float rc = key > 1u ? rcp_nr(c0) : 0.0f;  // a zero column eliminates nothing
+            const unsigned wk = __reduce_max_sync(0xffffffffu, key);
+            const unsigned bal = __ballot_sync(0xffffffffu, key == wk);
+            const bool me = key == wk && (bal & below) == 0u;
+            float4* cw = g.cand[b][warp];
 #pragma unroll
             for (int r = 0; r < kTsRpt; ++r) {
-                if (r == rbest) {
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        g.cand[b][warp][q] = make_float4(v[r][4 * q], v[r][4 * q + 1], v[r][4 * q + 2], v[r][4 * q + 3]);
-                }
+                st_if(me && rb == r, cw, v[r][0], v[r][1], v[r][2], v[r][3]);
+                st_if(me && rb == r, cw + 1, v[r][4], v[r][5], v[r][6], v[r][7]);
             }
-            g.cand[b][warp][8] = make_float4(rc, __uint_as_float((unsigned)(rbest * kTsThreads + t)), 0.f, 0.f);
-            atomicMax(&g.best[b3], ((wk > 8u ? wk : 8u) & ~7u) | (unsigned)(7 - warp));
-        }
-        __syncthreads();
-        const unsigned pk = g.best[b3];
-        if (t == 0) g.best[b3 == 0 ? 2 : b3 - 1] = 0u;  // the slot of column j + 2
-        b3 = b3 == 2 ? 0 : b3 + 1;
-        if (pk == 0u) break;  // no live row left anywhere (uniform)
-        const int pwarp = 7 - (int)(pk & 7u);
-        float pr[32];
+            st_if(me, cw + 2, rc, __uint_as_float((unsigned)(rb * kTsThreads + t)));
+            st_if(me, reinterpret_cast<unsigned*>(&g.key[b][0]) + warp,
+                  wk != 0u ? ((wk > 8u ? wk : 8u) & ~7u) | (unsigned)(7 - warp) : 0u);
+            __syncthreads();
+            const uint4 ka = g.key[b][0], kb = g.key[b][1];
+            const unsigned pk = max(max(max(ka.x, ka.y), max(ka.z, ka.w)), max(max(kb.x, kb.y), max(kb.z, kb.w)));
+            const float4* cp = g.cand[b][7 - (int)(pk & 7u)];
+            const float4 f0 = cp[0], f1 = cp[1];
+            const float2 meta = *reinterpret_cast<const float2*>(cp + 2);
+            const float pr[kTsBk] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
+            const int ps = (int)__float_as_uint(meta.y);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const float4 f = g.cand[b][pwarp][q];
-            pr[4 * q] = f.x; pr[4 * q + 1] = f.y; pr[4 * q + 2] = f.z; pr[4 * q + 3] = f.w;
+            for (int r = 0; r < kTsRpt; ++r) {
+                pq[r] = pq[r] == -1 && ps == r * kTsThreads + t ? jb + q : pq[r];
+                const float l = pq[r] == -1 ? v[r][0] * meta.x : 0.f;
+#pragma unroll
+                for (int k = 1; k < kTsBk; ++k) v[r][k - 1] = fmaf(-l, pr[k], v[r][k]);
+                v[r][kTsBk - 1] = 0.f;
+                mul[q * kTsRows + r * kTsThreads + t] = l;
+            }
+            if (lm && t < kTsBk - q) g.ur[jb + q][jb + q + t] = reinterpret_cast<const float*>(cp)[t];
         }
-        const float4 meta = g.cand[b][pwarp][8];
-        const float rcp = meta.x;
-        const unsigned ps = __float_as_uint(meta.y);
-        if (lm && t < 8) g.u[j][t] = g.cand[b][pwarp][t];
+        // the block's pivots: their place, and their rows right of the block
 #pragma unroll
         for (int r = 0; r < kTsRpt; ++r) {
-            if (ps == (unsigned)(r * kTsThreads + t)) {
-                live[r] = false;
-                s_win[j] = rid[r];
-                s_loc[j] = r * kTsThreads + t;
-            }
-            const float l = live[r] ? v[r][0] * rcp : 0.f;
-            if (lm) lm[j * kTsRows + r * kTsThreads + t] = l;
+            if (pq[r] < jb) continue;
+            s_win[pq[r]] = rid[r];
+            s_loc[pq[r]] = r * kTsThreads + t;
+            float* dst = g.u[pq[r] - jb];
 #pragma unroll
-            for (int k = 1; k < 32; ++k) v[r][k - 1] = fmaf(-l, pr[k], v[r][k]);
-            v[r][31] = 0.f;
+            for (int k = kTsBk; k < 32; k += 4)
+                *reinterpret_cast<float4*>(dst + k - kTsBk) = make_float4(v[r][k], v[r][k + 1], v[r][k + 2], v[r][k + 3]);
+        }
+        float l[kTsRpt][kTsBk];
+#pragma unroll
+        for (int r = 0; r < kTsRpt; ++r)
+#pragma unroll
+            for (int q = 0; q < kTsBk; ++q) {
+                l[r][q] = mul[q * kTsRows + r * kTsThreads + t];
+                if (lm) lm[(jb + q) * kTsRows + r * kTsThreads + t] = l[r][q];
+            }
+        const int c1 = jb + kTsBk;
+        if (c1 >= w) break;
+        __syncthreads();
+        if (t < 32 - kTsBk) {  // U right of the block
+            float x[kTsBk];
+#pragma unroll
+            for (int q = 0; q < kTsBk; ++q) x[q] = g.u[q][t];
+#pragma unroll
+            for (int q1 = 1; q1 < kTsBk; ++q1) {
+                const float* lp = mul + max(s_loc[jb + q1], 0);
+#pragma unroll
+                for (int q0 = 0; q0 < q1; ++q0) x[q1] = fmaf(-lp[q0 * kTsRows], x[q0], x[q1]);
+            }
+#pragma unroll
+            for (int q = 0; q < kTsBk; ++q) {
+                g.u[q][t] = x[q];
+                if (lm && c1 + t < 32) g.ur[jb + q][c1 + t] = x[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 32 - kTsBk; k += 4) {
+#pragma unroll
+            for (int r = 0; r < kTsRpt; ++r)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[r][k + e] = v[r][k + kTsBk + e];
+            if (c1 + k >= 32) continue;  // nothing left there
+#pragma unroll
+            for (int q = 0; q < kTsBk; ++q) {
+                const float4 uu = *reinterpret_cast<const float4*>(&g.u[q][k]);
+#pragma unroll
+                for (int r = 0; r < kTsRpt; ++r) {
+                    v[r][k] = fmaf(-l[r][q], uu.x, v[r][k]);
+                    v[r][k + 1] = fmaf(-l[r][q], uu.y, v[r][k + 1]);
+                    v[r][k + 2] = fmaf(-l[r][q], uu.z, v[r][k + 2]);
+                    v[r][k + 3] = fmaf(-l[r][q], uu.w, v[r][k + 3]);
+                }
+            }
         }
     }
     __syncthreads();
 }
 
-// loads columns [c0, c0 + w) of row `row` (zeros past w); rows are 128-byte aligned
-__device__ __forceinline__ void load_leaf_row(const float* A, int64_t ld, int row, int c0, int w, float (&x)[32]) {
-    if (row < 0) {
+// Loads columns [c0, c0 + w) (zeros past w) of every thread's rows, rid[r] (zeros where < 0): a warp reads
+// its rows 128 bytes at a time, eight lanes a row, and hands them to their threads through shared memory
+// (stage, a warp's own 32 rows of pitch 36).  A thread that read its own row touched 32 lines a load.
+constexpr int kTsPitch = 36;
+__device__ __forceinline__ void load_leaf_rows(const float* A, int64_t ld, const int (&rid)[kTsRpt], int c0, int w,
+                                               float* stage, float (&x)[kTsRpt][32]) {
+    const int lane = threadIdx.x & 31, sub = lane >> 3, ch = 4 * (lane & 7);
 #pragma unroll
-        for (int k = 0; k < 32; ++k) x[k] = 0.f;
-        return;
+    for (int r = 0; r < kTsRpt; ++r)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int row = __shfl_sync(0xffffffffu, rid[r], 4 * i + sub);
+            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (row >= 0) f = __ldg(reinterpret_cast<const float4*>(A + (int64_t)row * ld + c0 + ch));
+            x[r][4 * i] = f.x; x[r][4 * i + 1] = f.y; x[r][4 * i + 2] = f.z; x[r][4 * i + 3] = f.w;
+        }
+#pragma unroll
+    for (int r = 0; r < kTsRpt; ++r) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            *reinterpret_cast<float4*>(stage + (4 * i + sub) * kTsPitch + ch) =
+                make_float4(x[r][4 * i], x[r][4 * i + 1], x[r][4 * i + 2], x[r][4 * i + 3]);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float4 f = *reinterpret_cast<const float4*>(stage + lane * kTsPitch + 4 * q);
+            x[r][4 * q] = f.x; x[r][4 * q + 1] = f.y; x[r][4 * q + 2] = f.z; x[r][4 * q + 3] = f.w;
+        }
     }
-    const float4* p = reinterpret_cast<const float4*>(A + (int64_t)row * ld + c0);
+    if (w < 32) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const float4 f = __ldg(p + q);
-        x[4 * q + 0] = f.x; x[4 * q + 1] = f.y; x[4 * q + 2] = f.z; x[4 * q + 3] = f.w;
+        for (int r = 0; r < kTsRpt; ++r)
+#pragma unroll
+            for (int k = 0; k < 32; ++k)
+                if (k >= w) x[r][k] = 0.f;
     }
-#pragma unroll
-    for (int k = 0; k < 32; ++k)
-        if (k >= w) x[k] = 0.f;
 }
 
 __global__ void __launch_bounds__(kTsThreads) tslu_select_kernel(TsArgs a) {
     __shared__ __align__(16) GeppSmem s_g;
     __shared__ int s_win[32], s_loc[32];
-    __shared__ float s_lu[32][33];
-    __shared__ __align__(16) float s_lt[32][32];  // s_lt[j][k] = L(k, j) for k > j, else 0
-    __shared__ __align__(16) float s_ut[32][32];  // s_ut[i][k] = U(k, i) for k < i, else 0
+    __shared__ __align__(16) float s_buf[kTsWarps * 32 * kTsPitch];  // row staging, multipliers; at the root:
+    float (*s_lt)[32] = reinterpret_cast<float (*)[32]>(s_buf);         // s_lt[j][k] = L(k, j) for k > j, else 0
+    float (*s_ut)[32] = reinterpret_cast<float (*)[32]>(s_buf + 1024);  // s_ut[i][k] = U(k, i) for k < i, else 0
+    float (*s_lu)[33] = reinterpret_cast<float (*)[33]>(s_buf + 2048);
+    static_assert(sizeof(s_buf) >= kTsBk * kTsRows * sizeof(float), "a block's multipliers fit");
+    static_assert(sizeof(s_buf) >= (2048 + 32 * 33) * sizeof(float), "the root's triangles fit");
     __shared__ float s_rdiag[32];
     __shared__ int s_last, s_bad;
     __shared__ int s_flag[32], s_outpos[32], s_mdst[64], s_msrc[64], s_nm, s_nout;
-    if (a.status[kInfo] != 0) return;
     const int t = threadIdx.x;
     const int m = a.n - a.lc0;
+    const int info = a.status[kInfo];  // (checked below: its latency runs under the rows')
     float v[kTsRpt][32];
     int rid[kTsRpt];
 #pragma unroll
     for (int r = 0; r < kTsRpt; ++r) {
         const int row = a.lc0 + blockIdx.x * kTsRows + r * kTsThreads + t;
         rid[r] = row < a.n ? row : -1;
-        load_leaf_row(a.A, a.ld, rid[r], a.lc0, a.w, v[r]);
-        if (a.pmap && row < a.n) a.pmap[row] = row;
+    }
+    float* stage = s_buf + (t >> 5) * 32 * kTsPitch;
+    load_leaf_rows(a.A, a.ld, rid, a.lc0, a.w, stage, v);
+    if (info != 0) return;
+    if (a.pmap) {
+#pragma unroll
+        for (int r = 0; r < kTsRpt; ++r)
+            if (rid[r] >= 0) a.pmap[rid[r]] = rid[r];
     }
     int node = blockIdx.x, count = (int)ceil_div(m, kTsRows), level = 0;
     for (;;) {
-        block_gepp(v, rid, a.w, s_win, s_loc, s_g, count == 1 ? a.lmul : nullptr);
+        block_gepp(v, rid, a.w, s_win, s_loc, s_g, s_buf, count == 1 ? a.lmul : nullptr);
         if (count == 1) break;
         // publish this node's candidates; the last member of the group merges them
         if (t < 32) a.cand[((int64_t)level * kTsMaxCand + node) * 32 + t] = s_win[t];
@@ -228,8 +339,7 @@ __global__ void __launch_bounds__(kTsThreads) tslu_select_kernel(TsArgs a) {
                          ? __ldcg(a.cand + ((int64_t)level * kTsMaxCand + parent * kTsFan + mem) * 32 + (sidx & 31))
                          : -1;
         }
-#pragma unroll
-        for (int r = 0; r < kTsRpt; ++r) load_leaf_row(a.A, a.ld, rid[r], a.lc0, a.w, v[r]);
+        load_leaf_rows(a.A, a.ld, rid, a.lc0, a.w, stage, v);
         node = parent;
         count = (int)ceil_div(count, kTsFan);
         ++level;
@@ -246,9 +356,7 @@ __global__ void __launch_bounds__(kTsThreads) tslu_select_kernel(TsArgs a) {
                 if (k < j) {
                     x = __ldcg(a.lmul + k * kTsRows + l);
                 } else {
-                    const float4 f = s_g.u[j][(k - j) >> 2];
-                    const int e4 = (k - j) & 3;
-                    x = e4 == 0 ? f.x : e4 == 1 ? f.y : e4 == 2 ? f.z : f.w;
+                    x = s_g.ur[j][k];
                 }
             }
             return x;
@@ -826,10 +934,11 @@ int32_t lu_factor_f32(Ctx* ctx, cudaStream_t st, float* A, int64_t ld, int64_t n
     const int di_smem = 2 * kTrsvNB * (kTrsvNB + 1) * sizeof(float);
     if (!attr.load()) {
         B2M_CU(ctx, cudaFuncSetAttribute(lu_outer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ou_smem));
+        B2M_CU(ctx, cudaFuncSetAttribute(tslu_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTsReserve));
         B2M_CU(ctx, cudaFuncSetAttribute(diag_inv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, di_smem));
         B2M_CU(ctx, cudaFuncSetAttribute(coupling_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCpSmem));
-        // one shared-memory carveout for every kernel of the factorisation, so that the panel kernels
-        // can share SMs with the tiles of a concurrent trailing GEMM (which needs the maximum)
+        // one shared-memory carveout for every kernel of the factorisation, so that the apply kernel
+        // and the outer ones can share SMs with the tiles of a concurrent trailing GEMM (which needs the maximum)
         for (const void* f : {(const void*)tslu_select_kernel, (const void*)tslu_apply_kernel,
                               (const void*)panel_permute_kernel, (const void*)lu_outer_kernel})
             B2M_CU(ctx, cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -886,7 +995,7 @@ int32_t lu_factor_f32(Ctx* ctx, cudaStream_t st, float* A, int64_t ld, int64_t n
                           s.moves, s.lmul, lc0 == oc0 ? pmap : nullptr, lpinv, ctx->d_status};
                 prof_begin(ctx, q, kClsPanel);
                 {
-                    const cudaLaunchConfig_t c = cfg_of((unsigned)ceil_div(n - lc0, kTsRows), kTsThreads, 0);
+                    const cudaLaunchConfig_t c = cfg_of((unsigned)ceil_div(n - lc0, kTsRows), kTsThreads, kTsReserve);
                     B2M_CU(ctx, cudaLaunchKernelEx(&c, tslu_select_kernel, ta));
                 }
                 prof_end(ctx, q, kClsPanel, 4.0 * (n - lc0) * 32);  // bytes: the leaf's columns, read once
