@@ -625,9 +625,11 @@ template <int NW> __device__ __forceinline__ void lu_sync(int bar) {
 
 // Leaf of w <= W columns over m rows (loaded in s.S, zero past column w): eliminates with partial
 // pivoting.  pos[r] of row t + r * NW * 32 (its position on entry): its position afterwards, or
-// -1 - j for the pivot of column j.  Multipliers are left in S, U11 in s.u.  False: singular.
+// -1 - j for the pivot of column j.  Multipliers are left in S, U11 in s.u; ipiv (may be null): ipiv[j] = c0 + the
+// position column j's pivot row had.  False: singular.
 template <int NW, int W>
-__device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w, int m, int (&pos)[2]) {
+__device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w, int m, int (&pos)[2],
+                                        int32_t* ipiv = nullptr, int c0 = 0) {
     constexpr int NT = NW * 32, RPT = 2;
     const int lane = t & 31, warp = t >> 5;
     double* S = s.S;
@@ -727,7 +729,10 @@ __device__ __forceinline__ bool lu_leaf(LuSlice<NW, W>& s, int t, int bar, int w
             if (!(fabs(u[0]) > sing_thresh<double>())) return false;  // uniform: every warp read the same
             if (warp == NW - 1) {  // the pivot row's part of U inside its block
                 if (lane < kBk && q + lane < kBk && j + lane < W) s.u[j * W + j + lane] = b.row[lane];
-                if (lane == 0) s.pl[j] = pl.y;
+                if (lane == 0) {
+                    s.pl[j] = pl.y;
+                    if (ipiv) ipiv[j] = c0 + pl.x;
+                }
             }
 #pragma unroll
             for (int r = 0; r < RPT; ++r) {
@@ -829,17 +834,19 @@ __device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, doubl
 // (0, 1) counts rows 2 t + s.  So neither shared memory nor shuffles lie between the solve and the
 // updates; only the 8 x 8 triangles go by substitution, with a shuffle per row.  (A thread per column
 // read each multiplier by a broadcast, which costs the SM's shared memory 2 cycles per warp: 10,600
-// cycles a leaf of order 256.)
-template <int NW, int W, bool kFirst>
-__device__ __forceinline__ void lu_strip(LuSlice<NW, W>& s, int lane, const double* A, const double* B, int n, int kk,
-                                         int ld, double* V, int c0, int w, int q0) {
+// cycles a leaf of order 256.)  kSum: the trailing update's products are summed before they meet the old value
+// (as in the products of the larger orders' factorisation; a third of the rounding, but registers that three CTAs
+// an SM do not have).
+template <int NW, int W, bool kFirst, bool kSum = false>
+__device__ __forceinline__ void lu_strip(LuSlice<NW, W>& s, int lane, const double* A, int64_t lda, const double* B,
+                                         int n, int kk, int ld, double* V, int c0, int w, int q0) {
     const int g = lane >> 2, t = lane & 3, nt = n + kk, cb = c0 + w, mr = n - cb;
     auto sx = [](int row, int c) { return row * W + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
     // Element (row, col) as this step finds it: A and B before the first update (kFirst).  Columns past
     // the last one read it again, so that no load hides behind a branch; they are not stored.
     auto at = [&](int row, int col) {
         const int c = min(col, nt - 1);
-        if constexpr (kFirst) return c < n ? A[row * n + c] : B[row * kk + c - n];
+        if constexpr (kFirst) return c < n ? A[row * lda + c] : B[row * kk + c - n];
         else return V[row * ld + c];
     };
     double x[W / 8][4];
@@ -918,11 +925,14 @@ __device__ __forceinline__ void lu_strip(LuSlice<NW, W>& s, int lane, const doub
     fetch(0, ro);
 #pragma unroll 1
     for (int r0 = 0; r0 < mr; r0 += 16) {
-        double acc[2][4];
+        double acc[2][4], add[2][4];
 #pragma unroll
         for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[h][e] = old[h][e];
+            for (int e = 0; e < 4; ++e) {
+                acc[h][e] = kSum ? 0.0 : old[h][e];
+                add[h][e] = old[h][e];
+            }
         const int la = s.lrow[w + min(r0 + g, mr - 1)], lb = s.lrow[w + min(r0 + g + 8, mr - 1)];
         int rn[2] = {ro[0], ro[1]};
         if (r0 + 16 < mr) fetch(r0 + 16, rn);
@@ -936,6 +946,11 @@ __device__ __forceinline__ void lu_strip(LuSlice<NW, W>& s, int lane, const doub
                 dmma(acc[h], a0.y, a1.y, x[b][2 * h + 1]);
             }
         }
+        if constexpr (kSum)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[h][e] += add[h][e];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             double* dst = V + ro[e] * ld + q0 + 2 * t;
@@ -949,76 +964,12 @@ __device__ __forceinline__ void lu_strip(LuSlice<NW, W>& s, int lane, const doub
     }
 }
 
-// One system on a group of NW warps; V is its scratch (row stride ld, 16-byte aligned rows).  0, or 1
-// when singular (uniform over the group).
+// y <- U^-1 y (y: n x 8 in s.S), U in the rows V[s.perm[i]] (stride ld); a block of U goes to s.u.
 template <int NW, int W>
-__device__ __forceinline__ int lu_system(LuSlice<NW, W>& s, int t, int bar, const double* A, const double* B, double* X,
-                                         int n, int kk, double* V) {
+__device__ __forceinline__ void lu_upper(LuSlice<NW, W>& s, int t, int bar, const double* V, int64_t ld, int n) {
     constexpr int NT = NW * 32;
-    const int lane = t & 31, warp = t >> 5, ld = (n + kk + 1) & ~1, nt = n + kk;
-    auto sx = [](int row, int c) { return row * W + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
-    for (int i = t; i < n; i += NT) s.perm[i] = (uint16_t)i;
-    lu_sync<NW>(bar);
-    for (int c0 = 0; c0 < n; c0 += W) {
-        const bool first = c0 == 0;
-        const int w = min(W, n - c0), m = n - c0, cb = c0 + w;
-        if (first) {
-#pragma unroll 4
-            for (int e = t; e < m * W; e += NT) {
-                const int rl = e / W, c = e % W;
-                cp_async8(s.S + sx(rl, c), c < w ? A + (int64_t)rl * n + c : A, c < w ? 8 : 0);
-            }
-        } else {
-#pragma unroll 4
-            for (int e = t; e < m * (W / 2); e += NT) {
-                const int rl = e / (W / 2), c = 2 * (e % (W / 2));
-                cp_async16(s.S + sx(rl, c), c < w ? V + s.perm[c0 + rl] * ld + c0 + c : V,
-                           c + 1 < w ? 16 : (c < w ? 8 : 0));
-            }
-        }
-        cp_async_commit();
-        int pos[2], row[2];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int rl = t + r * NT;
-            pos[r] = rl < m ? rl : -1 - W;
-            row[r] = rl < m ? s.perm[c0 + rl] : 0;
-        }
-        cp_async_wait<0>();
-        lu_sync<NW>(bar);
-        if (!lu_leaf<NW, W>(s, t, bar, w, m, pos)) return 1;
-        lu_sync<NW>(bar);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int rl = t + r * NT;
-            if (rl < m) s.perm[c0 + (pos[r] < 0 ? -1 - pos[r] : pos[r])] = (uint16_t)row[r];
-            if (rl < m && pos[r] >= 0) s.lrow[pos[r]] = (uint16_t)rl;
-        }
-        lu_sync<NW>(bar);
-        for (int e0 = t; e0 < W * W; e0 += 4 * NT) {  // U11
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int e = e0 + i * NT, j = e / W, c = e % W;
-                if (j < w && c >= j && c < w) V[s.perm[c0 + j] * ld + c0 + c] = s.u[e];
-            }
-        }
-        // the columns to the right, 16 a warp (strips of 32 took 10.5 ms instead of 8.8: more registers
-        // than three CTAs an SM allow, and idle warps on the last columns)
-        auto strips = [&](auto first) {
-            constexpr bool kFirst = decltype(first)::value;
-            for (int q0 = cb + 16 * warp; q0 < nt; q0 += 16 * NW)
-                lu_strip<NW, W, kFirst>(s, lane, A, B, n, kk, ld, V, c0, w, q0);
-        };
-        if (first) strips(std::true_type{});
-        else strips(std::false_type{});
-        lu_sync<NW>(bar);
-    }
-    // ---- back substitution: y (n x 8, zero past kk) in S's place, a block of U in u
+    const int lane = t & 31, warp = t >> 5;
     double* y = s.S;
-    for (int e = t; e < n * kBMaxK; e += NT) {
-        const int j = e / kBMaxK, q = e % kBMaxK;
-        y[e] = q < kk ? V[s.perm[j] * ld + n + q] : 0.0;
-    }
     for (int b0 = (n - 1) / W * W; b0 >= 0; b0 -= W) {
         const int bs = min(W, n - b0);
         lu_sync<NW>(bar);
@@ -1095,7 +1046,7 @@ __device__ __forceinline__ int lu_system(LuSlice<NW, W>& s, int t, int bar, cons
         // fold the block into the rows above (only full blocks of 4 k: bs < W only in the last one)
         const int g = lane >> 2, tq = lane & 3;
         for (int r0 = 16 * warp; r0 < b0; r0 += 16 * NW) {
-            const int ra = s.perm[r0 + g] * ld + b0, rb = s.perm[r0 + g + 8] * ld + b0;  // (b0 is a multiple of 16)
+            const int64_t ra = s.perm[r0 + g] * ld + b0, rb = s.perm[r0 + g + 8] * ld + b0;  // (b0 is a multiple of 16)
             double a0[W / 4], a1[W / 4], acc[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
             for (int k = 0; k < W / 4; ++k) {
@@ -1117,6 +1068,79 @@ __device__ __forceinline__ int lu_system(LuSlice<NW, W>& s, int t, int bar, cons
             *yb = make_double2(yb->x - acc[2], yb->y - acc[3]);
         }
     }
+}
+
+// One system on a group of NW warps; V is its scratch (row stride ld, 16-byte aligned rows).  0, or 1
+// when singular (uniform over the group).
+template <int NW, int W>
+__device__ __forceinline__ int lu_system(LuSlice<NW, W>& s, int t, int bar, const double* A, const double* B, double* X,
+                                         int n, int kk, double* V) {
+    constexpr int NT = NW * 32;
+    const int lane = t & 31, warp = t >> 5, ld = (n + kk + 1) & ~1, nt = n + kk;
+    auto sx = [](int row, int c) { return row * W + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
+    for (int i = t; i < n; i += NT) s.perm[i] = (uint16_t)i;
+    lu_sync<NW>(bar);
+    for (int c0 = 0; c0 < n; c0 += W) {
+        const bool first = c0 == 0;
+        const int w = min(W, n - c0), m = n - c0, cb = c0 + w;
+        if (first) {
+#pragma unroll 4
+            for (int e = t; e < m * W; e += NT) {
+                const int rl = e / W, c = e % W;
+                cp_async8(s.S + sx(rl, c), c < w ? A + (int64_t)rl * n + c : A, c < w ? 8 : 0);
+            }
+        } else {
+#pragma unroll 4
+            for (int e = t; e < m * (W / 2); e += NT) {
+                const int rl = e / (W / 2), c = 2 * (e % (W / 2));
+                cp_async16(s.S + sx(rl, c), c < w ? V + s.perm[c0 + rl] * ld + c0 + c : V,
+                           c + 1 < w ? 16 : (c < w ? 8 : 0));
+            }
+        }
+        cp_async_commit();
+        int pos[2], row[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int rl = t + r * NT;
+            pos[r] = rl < m ? rl : -1 - W;
+            row[r] = rl < m ? s.perm[c0 + rl] : 0;
+        }
+        cp_async_wait<0>();
+        lu_sync<NW>(bar);
+        if (!lu_leaf<NW, W>(s, t, bar, w, m, pos)) return 1;
+        lu_sync<NW>(bar);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int rl = t + r * NT;
+            if (rl < m) s.perm[c0 + (pos[r] < 0 ? -1 - pos[r] : pos[r])] = (uint16_t)row[r];
+            if (rl < m && pos[r] >= 0) s.lrow[pos[r]] = (uint16_t)rl;
+        }
+        lu_sync<NW>(bar);
+        for (int e0 = t; e0 < W * W; e0 += 4 * NT) {  // U11
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int e = e0 + i * NT, j = e / W, c = e % W;
+                if (j < w && c >= j && c < w) V[s.perm[c0 + j] * ld + c0 + c] = s.u[e];
+            }
+        }
+        // the columns to the right, 16 a warp (strips of 32 took 10.5 ms instead of 8.8: more registers
+        // than three CTAs an SM allow, and idle warps on the last columns)
+        auto strips = [&](auto first) {
+            constexpr bool kFirst = decltype(first)::value;
+            for (int q0 = cb + 16 * warp; q0 < nt; q0 += 16 * NW)
+                lu_strip<NW, W, kFirst>(s, lane, A, n, B, n, kk, ld, V, c0, w, q0);
+        };
+        if (first) strips(std::true_type{});
+        else strips(std::false_type{});
+        lu_sync<NW>(bar);
+    }
+    // ---- back substitution: y (n x 8, zero past kk) in S's place, a block of U in u
+    double* y = s.S;
+    for (int e = t; e < n * kBMaxK; e += NT) {
+        const int j = e / kBMaxK, q = e % kBMaxK;
+        y[e] = q < kk ? V[s.perm[j] * ld + n + q] : 0.0;
+    }
+    lu_upper<NW, W>(s, t, bar, V, ld, n);
     lu_sync<NW>(bar);
     for (int e = t; e < n * kk; e += NT) X[e] = y[e / kk * kBMaxK + e % kk];
     lu_sync<NW>(bar);
@@ -1175,6 +1199,195 @@ __global__ void __launch_bounds__(kLuThreads, kLuCtas) batch_lu_kernel(BatchArgs
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// One system of order <= 256 in the calls on a single matrix: its factorisation in place (small_lu_kernel)
+// and the solves with its factors (small_solve_kernel), one launch each, on the parts above.  The recursion of
+// the larger orders needs four launches a leaf here (panel, interchanges, U12, update), each shorter than
+// the gap to the next; its solve a copy, a gather and two sweeps.
+//
+// small_lu_kernel: four warps do the leaves, eight the strips.  L is kept too, in its storage row; rows go to
+// their positions at the end, from the scratch V (n rows of (n + 1) & ~1) back to A.
+// Measured on a B200 (factor and one right-hand side, the whole call): order 100 201 us before and 126 us now,
+// order 256 429 and 350 us; the inverse of order 100 230 and 129 us.
+// ------------------------------------------------------------------------------------------
+constexpr int kSmThreads = 256;
+
+__global__ void __launch_bounds__(kSmThreads, 1)
+    small_lu_kernel(double* A, int64_t ld, int n, double* V, int32_t* ipiv, int32_t* perm, int32_t* status) {
+    constexpr int W = 32;
+    extern __shared__ __align__(16) unsigned char lu_dyn[];
+    LuSlice<4, W>& s = *reinterpret_cast<LuSlice<4, W>*>(lu_dyn);
+    __shared__ int16_t s_pos[kBMaxN];   // of a leaf's rows: position (-1 - j: the pivot of column j),
+    __shared__ uint16_t s_row[kBMaxN];  // storage row
+    __shared__ int s_stop;
+    if (status[kInfo] != 0) return;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, ldv = (n + 1) & ~1;
+    auto sx = [](int row, int c) { return row * W + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
+    for (int i = t; i < n; i += kSmThreads) s.perm[i] = (uint16_t)i;
+    if (t == 0) s_stop = 0;
+    __syncthreads();
+    for (int c0 = 0; c0 < n; c0 += W) {
+        const bool first = c0 == 0;
+        const int w = min(W, n - c0), m = n - c0, cb = c0 + w;
+        if (first) {
+#pragma unroll 4
+            for (int e = t; e < m * W; e += kSmThreads) {
+                const int rl = e / W, c = e % W;
+                cp_async8(s.S + sx(rl, c), c < w ? A + rl * ld + c : A, c < w ? 8 : 0);
+            }
+        } else {
+#pragma unroll 4
+            for (int e = t; e < m * (W / 2); e += kSmThreads) {
+                const int rl = e / (W / 2), c = 2 * (e % (W / 2));
+                cp_async16(s.S + sx(rl, c), c < w ? V + s.perm[c0 + rl] * ldv + c0 + c : V,
+                           c + 1 < w ? 16 : (c < w ? 8 : 0));
+            }
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+        if (t < 128) {
+            int pos[2], row[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int rl = t + r * 128;
+                pos[r] = rl < m ? rl : -1 - W;
+                row[r] = rl < m ? s.perm[c0 + rl] : 0;
+            }
+            const bool ok = lu_leaf<4, W>(s, t, 1, w, m, pos, ipiv + c0, c0);
+            if (!ok && t == 0) {
+                s_stop = 1;
+                atomicExch(&status[kInfo], 1);
+            }
+            lu_sync<4>(1);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int rl = t + r * 128;
+                if (!ok || rl >= m) continue;
+                s.perm[c0 + (pos[r] < 0 ? -1 - pos[r] : pos[r])] = (uint16_t)row[r];
+                if (pos[r] >= 0) s.lrow[pos[r]] = (uint16_t)rl;
+                s_pos[rl] = (int16_t)pos[r];
+                s_row[rl] = (uint16_t)row[r];
+            }
+        }
+        __syncthreads();
+        if (s_stop) return;
+        for (int e = t; e < m * (W / 2); e += kSmThreads) {  // the leaf's columns
+            const int rl = e / (W / 2), c = 2 * (e % (W / 2)), j = -1 - s_pos[rl];
+            double2 x = *reinterpret_cast<const double2*>(s.S + sx(rl, c));
+            if (j >= 0) {
+                const double2 u = *reinterpret_cast<const double2*>(s.u + j * W + c);
+                x = make_double2(c >= j ? u.x : x.x, c + 1 >= j ? u.y : x.y);
+            }
+            if (c < w) *reinterpret_cast<double2*>(V + s_row[rl] * ldv + c0 + c) = x;
+        }
+        auto strips = [&](auto first) {
+            for (int q0 = cb + 16 * warp; q0 < n; q0 += 16 * (kSmThreads / 32))
+                lu_strip<4, W, decltype(first)::value, true>(s, lane, A, ld, nullptr, n, 0, ldv, V, c0, w, q0);
+        };
+        if (first) strips(std::true_type{});
+        else strips(std::false_type{});
+        __syncthreads();
+    }
+    if (perm)
+        for (int i = t; i < n; i += kSmThreads) perm[i] = s.perm[i];
+    constexpr int B = 4;
+    for (int i0 = warp; i0 < n; i0 += B * (kSmThreads / 32))
+        for (int c = lane; c < n; c += 32) {
+            double v[B];
+#pragma unroll
+            for (int q = 0; q < B; ++q) v[q] = V[s.perm[min(i0 + q * (kSmThreads / 32), n - 1)] * ldv + c];
+#pragma unroll
+            for (int q = 0; q < B; ++q)
+                if (i0 + q * (kSmThreads / 32) < n) A[(i0 + q * (kSmThreads / 32)) * ld + c] = v[q];
+        }
+}
+
+// B <- U^-1 L^-1 P B, eight right-hand sides a CTA: in shared memory, blocks of 32 rows substituted by one
+// warp (lane = right-hand side + 8 * (row & 3)) and folded into the others on the FP64 tensor cores.
+__global__ void __launch_bounds__(128) small_solve_kernel(const double* LU, int64_t ld, int n, const int32_t* perm,
+                                                          double* B, int64_t ldb, int nrhs, const int32_t* status) {
+    constexpr int NW = 4, W = 32, NT = 128;
+    extern __shared__ __align__(16) unsigned char lu_dyn[];
+    LuSlice<NW, W>& s = *reinterpret_cast<LuSlice<NW, W>*>(lu_dyn);
+    if (status[kInfo] != 0) return;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int q0 = blockIdx.x * kBMaxK, kk = min(kBMaxK, nrhs - q0);
+    double* y = s.S;
+    for (int i = t; i < n; i += NT) s.perm[i] = (uint16_t)i;
+    for (int e = t; e < n * kBMaxK; e += NT) {
+        const int j = e / kBMaxK, q = e % kBMaxK;
+        y[e] = q < kk ? B[perm[j] * ldb + q0 + q] : 0.0;
+    }
+    for (int b0 = 0; b0 < n; b0 += W) {
+        const int bs = min(W, n - b0);
+        __syncthreads();
+        batched_copy<NT, 8, double>(t, W * W,  // the block's columns: u[c][r] = L(b0 + r, b0 + c), r > c
+            [&](int e) {
+                const int r = e / W, c = e % W;
+                return (r > c && r < bs) ? LU[(b0 + r) * ld + b0 + c] : 0.0;
+            },
+            [&](int e, double v) { s.u[e % W * W + e / W] = v; });
+        __syncthreads();
+        if (warp == 0) {
+            const int q = lane & 7, rg = lane >> 3;
+            double x[W / 4];
+#pragma unroll
+            for (int i = 0; i < W / 4; ++i) x[i] = 4 * i + rg < bs ? y[(b0 + 4 * i + rg) * kBMaxK + q] : 0.0;
+#pragma unroll 1
+            for (int i4 = 0; i4 < W / 4; ++i4) {
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    const double xj = __shfl_sync(0xffffffffu, x[0], q + 8 * v);
+                    const double* uc = &s.u[(4 * i4 + v) * W + 4 * i4 + rg];
+                    if (rg > v) x[0] = fma(-uc[0], xj, x[0]);
+#pragma unroll
+                    for (int i = 1; i < W / 4; ++i)
+                        if (i4 + i < W / 4) x[i] = fma(-uc[4 * i], xj, x[i]);
+                }
+                if (4 * i4 + rg < bs) y[(b0 + 4 * i4 + rg) * kBMaxK + q] = x[0];
+#pragma unroll
+                for (int i = 1; i < W / 4; ++i) x[i - 1] = x[i];
+            }
+        }
+        __syncthreads();
+        // the rows below (there are some only below a full block)
+        const int g = lane >> 2, tq = lane & 3;
+        for (int r0 = b0 + W + 16 * warp; r0 < n; r0 += 16 * NW) {
+            const int ra = min(r0 + g, n - 1), rb = min(r0 + g + 8, n - 1);
+            double a0[W / 4], a1[W / 4], acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < W / 4; ++k) {
+                a0[k] = LU[ra * ld + b0 + 4 * k + tq];
+                a1[k] = LU[rb * ld + b0 + 4 * k + tq];
+            }
+#pragma unroll
+            for (int k = 0; k < W / 4; ++k) dmma(acc, a0[k], a1[k], y[(b0 + 4 * k + tq) * kBMaxK + g]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (r0 + g + 8 * e >= n) continue;
+                double2* yp = reinterpret_cast<double2*>(y + (r0 + g + 8 * e) * kBMaxK + 2 * tq);
+                *yp = make_double2(yp->x - acc[2 * e], yp->y - acc[2 * e + 1]);
+            }
+        }
+    }
+    lu_upper<NW, W>(s, t, 1, LU, ld, n);
+    __syncthreads();
+    for (int e = t; e < n * kBMaxK; e += NT) {
+        const int j = e / kBMaxK, q = e % kBMaxK;
+        if (q < kk) B[j * ldb + q0 + q] = y[e];
+    }
+}
+
+template <typename Kern> int32_t small_attr(Ctx* ctx, Kern kern) {
+    std::atomic<int>& attr = device_flag((const void*)kern, 0, ctx->device);
+    if (!attr.load()) {
+        B2M_CU(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LuSlice<4, 32>)));
+        attr.store(1);
+    }
+    return B2M_OK;
+}
+
 size_t batch_smem_bytes(int small_n, int G, int pw_large, int pw_small, int GB) {
     const size_t big = slice_doubles(kBMaxN, pw_large) * ((kBThreads / 32) / GB);
     const size_t small = slice_doubles(small_n, pw_small) * ((kBThreads / 32) / G);
@@ -1182,6 +1395,29 @@ size_t batch_smem_bytes(int small_n, int G, int pw_large, int pw_small, int GB) 
 }
 
 }  // namespace
+
+size_t small_lu_scratch(int64_t n) { return (size_t)(n * ((n + 1) & ~(int64_t)1)) * sizeof(double); }
+
+int32_t small_lu_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t n, double* V, int32_t* ipiv,
+                     int32_t* perm) {
+    B2M_TRY(small_attr(ctx, small_lu_kernel));
+    prof_begin(ctx, st, kClsPanel);
+    small_lu_kernel<<<1, kSmThreads, sizeof(LuSlice<4, 32>), st>>>(A, ld, (int)n, V, ipiv, perm, ctx->d_status);
+    prof_end(ctx, st, kClsPanel, 16.0 * n * n);
+    B2M_LAUNCHED(ctx);
+    return B2M_OK;
+}
+
+int32_t small_solve_f64(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld, int64_t n, const int32_t* perm,
+                        double* B, int64_t ldb, int64_t nrhs) {
+    B2M_TRY(small_attr(ctx, small_solve_kernel));
+    prof_begin(ctx, st, kClsSolve);
+    small_solve_kernel<<<(unsigned)ceil_div(nrhs, kBMaxK), 128, sizeof(LuSlice<4, 32>), st>>>(
+        LU, ld, (int)n, perm, B, ldb, (int)nrhs, ctx->d_status);
+    prof_end(ctx, st, kClsSolve, 0.0);
+    B2M_LAUNCHED(ctx);
+    return B2M_OK;
+}
 
 // ------------------------------------------------------------------ host side
 struct BatchPlanCache {

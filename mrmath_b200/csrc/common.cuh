@@ -116,6 +116,7 @@ struct Ctx {
     int64_t launches = 0;
     Prof prof;
     bool use_graphs = true;
+    bool fixed_scratch = false;  // the allocation-free entry point: no workspace may be asked for
     std::map<GraphKey, GraphEntry> graphs;
     uint64_t graph_clock = 0;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

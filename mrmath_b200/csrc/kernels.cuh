@@ -105,6 +105,15 @@ int32_t z_determinant(Ctx* ctx, cudaStream_t st, const double* re, const double*
 // Builds perm from ipiv on the device (used when factors come from outside: b2m_MatrixLUBackSubst).
 int32_t perm_from_ipiv(Ctx* ctx, cudaStream_t st, const int32_t* ipiv, int64_t n, int32_t* perm);
 
+// One matrix of order n <= kSmallLu in one launch each (batched.cu): lu_factor_f64 with the scratch V of
+// small_lu_scratch(n) bytes, and lu_solve_f64.
+constexpr int64_t kSmallLu = 256;
+size_t small_lu_scratch(int64_t n);
+int32_t small_lu_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t n, double* V, int32_t* ipiv,
+                     int32_t* perm);
+int32_t small_solve_f64(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld, int64_t n, const int32_t* perm,
+                        double* B, int64_t ldb, int64_t nrhs);
+
 // Determinant from factors: (-1)^{#i: ipiv[i] != i} * prod diag, in the reference's order.
 int32_t lu_determinant(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld, int64_t n, const int32_t* ipiv,
                        double* d_det);

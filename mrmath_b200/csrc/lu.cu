@@ -1165,16 +1165,24 @@ int32_t lu_factor_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t 
         ctx->progress_notes.clear();
         ctx->progress_notes.reserve((size_t)(n / 8 + 2));
     }
-    // orders above 2 outer panels take the blocked look-ahead driver (row maps in a workspace); smaller
-    // ones (and every call of the allocation-free entry point, n <= 512) the plain recursion
-    const bool blocked = n > 2 * kOuterNB;
-    int32_t* pmap2 = nullptr;
-    if (blocked) {
-        void* p = nullptr;
-        B2M_TRY(ws_get(ctx, kWsPmap, (size_t)(2 * round_up(n, 64) + 2 * kPanelMoves) * sizeof(int32_t), &p));
-        pmap2 = static_cast<int32_t*>(p);
+    // Three ways, by the order (measured, factor + solve of one right-hand side, us):
+    //   * up to 256 (kSmallLu), one launch of one CTA (order 16: 36 against 44 by the recursion, 100: 126 / 201,
+    //     256: 350 / 429 and about 375 by the blocked driver);
+    //   * above, the blocked look-ahead driver with linked leaves (257: 377 / 491, 512: 658 / 931);
+    //   * the plain recursion where no workspace or side stream may be used (the allocation-free entry
+    //     point, n <= 512), and up to order 512 with progress reports, which it makes leaf by leaf.
+    // Every order asks for the small orders' scratch and the side streams, so that after a call of any order
+    // a smaller one allocates nothing (and can be captured).
+    const bool plain = ctx->fixed_scratch || (ctx->progress && n <= 2 * kOuterNB);
+    const bool blocked = !plain && n > kSmallLu;
+    void* scratch = nullptr;
+    if (!ctx->fixed_scratch) {
+        const size_t maps = (size_t)(2 * round_up(n, 64) + 2 * kPanelMoves) * sizeof(int32_t);
+        B2M_TRY(ws_get(ctx, kWsPmap, std::max(maps, small_lu_scratch(kSmallLu)), &scratch));
         B2M_TRY(ensure_side_stream(ctx));
     }
+    if (!plain && !blocked) return small_lu_f64(ctx, st, A, ld, n, static_cast<double*>(scratch), ipiv, perm);
+    int32_t* pmap2 = static_cast<int32_t*>(scratch);
     const GraphKey key{1, A, ipiv, perm, ctx->d_status, ld, n, 0, 0};
     const GraphKey key1{1, A, ipiv, perm, ctx->d_status, ld, n, 0, 1};
     B2M_TRY(run_graph(ctx, st, key, [&](cudaStream_t s) -> int32_t {
@@ -1195,6 +1203,9 @@ int32_t lu_solve_f64(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld, in
                      double* B, int64_t ldb, int64_t nrhs, double* tmp) {
     if (n <= 0 || nrhs <= 0) return B2M_OK;
     if ((ldb & 1) || !aligned16(B)) return fail(ctx, B2M_ERR_DIM, "lu_solve_f64: ldb must be even");
+    // (order 16, one right-hand side: 18 us against 23 by a copy, a gather and two sweeps, 100: 40 / 50, 256: 79 / 89;
+    // 256 right-hand sides 91 / 212)
+    if (n <= kSmallLu) return small_solve_f64(ctx, st, LU, ld, n, perm, B, ldb, nrhs);
     // X = P B
     double* X = tmp;
     if (!X) {
