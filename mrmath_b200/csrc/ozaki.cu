@@ -431,63 +431,139 @@ __device__ __forceinline__ int exp_of(double m) {
     return e;
 }
 
-// row exponents of A (M x K, row stride lda): one warp per row
-__global__ void ozaki_row_exp_kernel(const double* A, int64_t lda, int M, int K, int32_t* ea) {
-    const int row = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (row >= M) return;
-    double m = 0.0;
-    for (int k = lane; k < K; k += 32) m = fmax(m, fabs(A[(int64_t)row * lda + k]));
+// The slices of four scaled entries, a byte each: word[p] holds slice p of all four.  The first
+// eight slices of |x| < 1 are the 7-bit digits of trunc(|x| 2^56), so one conversion to an integer and
+// shifts replace the truncation, subtraction and conversion of every slice (FP64 conversions run at a
+// quarter of the rate; at order 8192 A's rows took 587 us with their exponents and take 215 now, B's
+// columns 386 and 244).  x 2^56 minus its integer part is
+// exact and gives the slices after the eighth.  An entry that is not below 1 in magnitude (no finite
+// exponent) takes the defining steps.
+template <typename Put>
+__device__ __forceinline__ void slice4(const double (&x)[4], int s, Put put) {
+    unsigned long long mag[4];
+    double rest[4];
+    uint32_t neg = 0;
+    bool odd = false;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) ea[row] = exp_of(m);
+    for (int e = 0; e < 4; ++e) {
+        const double y = fabs(x[e]) * 0x1.0p56;
+        odd = odd || !(y < 0x1.0p56);
+        mag[e] = (unsigned long long)__double2ll_rz(y);
+        rest[e] = y - (double)(long long)mag[e];
+        neg |= __double2hiint(x[e]) < 0 ? 0xffu << (8 * e) : 0u;
+    }
+    if (odd) {
+        double v[4] = {x[0], x[1], x[2], x[3]};
+        for (int p = 0; p < s; ++p) {
+            uint32_t word = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                v[e] *= 128.0;
+                const double d = trunc(v[e]);
+                v[e] -= d;
+                word |= (uint32_t)(uint8_t)(int8_t)d << (8 * e);
+            }
+            put(p, word);
+        }
+        return;
+    }
+    // a byte's negative -d, 0 <= d < 128, is (0x80 - d) ^ 0x80: no borrow leaves the byte
+    auto signed_bytes = [&](uint32_t w) { return (w & ~neg) | (((0x80808080u - w) ^ 0x80808080u) & neg); };
+    auto gather = [&](int sh) {
+        uint32_t d[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[e] = (uint32_t)(mag[e] >> sh);
+        return __byte_perm(__byte_perm(d[0], d[1], 0x0040), __byte_perm(d[2], d[3], 0x0040), 0x5410) & 0x7f7f7f7fu;
+    };
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+        if (p < s) put(p, signed_bytes(gather(7 * (7 - p))));
+    if (s <= 8) return;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) mag[e] = (unsigned long long)__double2ll_rz(rest[e] * 0x1.0p56);
+    for (int p = 8; p < s; ++p) put(p, signed_bytes(gather(7 * (15 - p))));
 }
 
-// column exponents of B (K x N, row stride ldb): a thread per column
-__global__ void ozaki_col_exp_kernel(const double* B, int64_t ldb, int K, int N, int32_t* eb) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= N) return;
+// Exponent and slices of A's rows (M x K, row stride lda), a CTA per row: A8[p][i][k] (p < s, row stride
+// Kp bytes).  The second pass over the row reads it from the L2.
+constexpr int kOzSliceThreads = 256;
+__global__ void __launch_bounds__(kOzSliceThreads) ozaki_slice_a_kernel(const double* A, int64_t lda, int M, int K,
+                                                                        int32_t* ea, int s, int8_t* A8, int64_t Kp) {
+    __shared__ double s_m[kOzSliceThreads / 32];
+    const int i = blockIdx.x, t = threadIdx.x;
+    const double* row = A + (int64_t)i * lda;
     double m = 0.0;
-    for (int k = 0; k < K; ++k) m = fmax(m, fabs(B[(int64_t)k * ldb + col]));
+#pragma unroll 8
+    for (int k = t; k < K; k += kOzSliceThreads) m = fmax(m, fabs(row[k]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((t & 31) == 0) s_m[t >> 5] = m;
+    __syncthreads();
+    m = s_m[0];
+#pragma unroll
+    for (int w = 1; w < kOzSliceThreads / 32; ++w) m = fmax(m, s_m[w]);
+    const int ex = exp_of(m);
+    if (t == 0) ea[i] = ex;
+    const double f = ldexp(1.0, -ex);
+#pragma unroll 2
+    for (int k = 4 * t; k < (int)Kp; k += 4 * kOzSliceThreads) {
+        double x[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = k + e < K ? row[k + e] * f : 0.0;
+        slice4(x, s, [&](int p, uint32_t w) {
+            *reinterpret_cast<uint32_t*>(A8 + ((int64_t)p * M + i) * Kp + k) = w;
+        });
+    }
+}
+
+// Column exponents of B (K x N, row stride ldb): a CTA per 32 columns, a warp per row of them.  110 us at order
+// 8192 (a thread per column took 890, 32 of the chip's 148 SMs busy).
+constexpr int kOzColThreads = 1024;
+__global__ void __launch_bounds__(kOzColThreads) ozaki_col_exp_kernel(const double* B, int64_t ldb, int K, int N,
+                                                                      int32_t* eb) {
+    __shared__ double s_m[kOzColThreads / 32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
+    double m = 0.0;
+    if (col < N) {
+#pragma unroll 8
+        for (int k = warp; k < K; k += kOzColThreads / 32) m = fmax(m, fabs(B[(int64_t)k * ldb + col]));
+    }
+    s_m[warp][lane] = m;
+    __syncthreads();
+    if (warp != 0 || col >= N) return;
+    for (int w = 1; w < kOzColThreads / 32; ++w) m = fmax(m, s_m[w][lane]);
     eb[col] = exp_of(m);
 }
 
-// A slices: A8[p][i][k] (p < s, row stride Kp bytes)
-__global__ void ozaki_slice_a_kernel(const double* A, int64_t lda, int M, int K, const int32_t* ea, int s,
-                                     int8_t* A8, int64_t Kp) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (int64_t)M * Kp) return;
-    const int i = (int)(e / Kp), k = (int)(e - (int64_t)i * Kp);
-    double x = k < K ? A[(int64_t)i * lda + k] * ldexp(1.0, -ea[i]) : 0.0;
-    for (int p = 0; p < s; ++p) {
-        x *= 128.0;
-        const double v = trunc(x);
-        x -= v;
-        A8[((int64_t)p * M + i) * Kp + k] = (int8_t)v;
+// B's slices, transposed to K-major: B8[q][j][k] (row stride Kp bytes), tiles of 128 rows x 32 columns
+// through shared memory, so that reads (along j) and writes (along k) are whole lines.
+constexpr int kOzTk = 128;
+__global__ void __launch_bounds__(kOzSliceThreads) ozaki_slice_b_kernel(const double* B, int64_t ldb, int K, int N,
+                                                                        const int32_t* eb, int s, int8_t* B8,
+                                                                        int64_t Kp) {
+    __shared__ double tile[32][kOzTk + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int k0 = blockIdx.y * kOzTk, j0 = blockIdx.x * 32;
+    const double f = j0 + lane < N ? ldexp(1.0, -eb[j0 + lane]) : 0.0;
+    constexpr int R = kOzTk / (kOzSliceThreads / 32);
+    double v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const int k = k0 + warp + i * (kOzSliceThreads / 32);
+        v[i] = k < K && j0 + lane < N ? B[(int64_t)k * ldb + j0 + lane] * f : 0.0;
     }
-}
-
-// B slices, transposed to K-major: B8[q][j][k] (row stride Kp bytes); 32 x 32 tiles through
-// shared memory so that both the read (along j) and the write (along k) are coalesced
-__global__ void ozaki_slice_b_kernel(const double* B, int64_t ldb, int K, int N, const int32_t* eb, int s,
-                                     int8_t* B8, int64_t Kp) {
-    __shared__ double tile[32][33];
-    const int k0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
-    const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-    for (int r = ty; r < 32; r += 8) {
-        const int k = k0 + r, j = j0 + tx;
-        tile[r][tx] = (k < K && j < N) ? B[(int64_t)k * ldb + j] * ldexp(1.0, -eb[j]) : 0.0;
-    }
+#pragma unroll
+    for (int i = 0; i < R; ++i) tile[lane][warp + i * (kOzSliceThreads / 32)] = v[i];
     __syncthreads();
-    for (int r = ty; r < 32; r += 8) {
-        const int j = j0 + r, k = k0 + tx;
-        if (j >= N || k >= Kp) continue;
-        double x = tile[tx][r];
-        for (int q = 0; q < s; ++q) {
-            x *= 128.0;
-            const double v = trunc(x);
-            x -= v;
-            B8[((int64_t)q * N + j) * Kp + k] = (int8_t)v;
-        }
+    for (int c = warp; c < 32; c += kOzSliceThreads / 32) {
+        const int j = j0 + c, k = k0 + 4 * lane;
+        if (j >= N) break;
+        double x[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = tile[c][4 * lane + e];
+        slice4(x, s, [&](int q, uint32_t w) {
+            *reinterpret_cast<uint32_t*>(B8 + ((int64_t)q * N + j) * Kp + k) = w;
+        });
     }
 }
 
@@ -517,14 +593,13 @@ int32_t ozaki_gemm(Ctx* ctx, cudaStream_t st, const double* A, int64_t lda, cons
     int32_t* eb = ea + M;
     int8_t* A8 = (int8_t*)pa;
     int8_t* B8 = (int8_t*)pb;
-    ozaki_row_exp_kernel<<<(unsigned)ceil_div(M, 8), 256, 0, st>>>(A, lda, (int)M, (int)K, ea);
-    B2M_LAUNCHED(ctx);
-    ozaki_col_exp_kernel<<<(unsigned)ceil_div(N, 256), 256, 0, st>>>(B, ldb, (int)K, (int)N, eb);
+    ozaki_col_exp_kernel<<<(unsigned)ceil_div(N, 32), kOzColThreads, 0, st>>>(B, ldb, (int)K, (int)N, eb);
     B2M_LAUNCHED(ctx);
     prof_begin(ctx, st, kClsOther);
-    ozaki_slice_a_kernel<<<(unsigned)ceil_div(M * Kp, 256), 256, 0, st>>>(A, lda, (int)M, (int)K, ea, s, A8, Kp);
-    dim3 gb((unsigned)ceil_div(N, 32), (unsigned)ceil_div(Kp, 32));
-    ozaki_slice_b_kernel<<<gb, dim3(32, 8), 0, st>>>(B, ldb, (int)K, (int)N, eb, s, B8, Kp);
+    ozaki_slice_a_kernel<<<(unsigned)M, kOzSliceThreads, 0, st>>>(A, lda, (int)M, (int)K, ea, s, A8, Kp);
+    B2M_LAUNCHED(ctx);
+    dim3 gb((unsigned)ceil_div(N, 32), (unsigned)(Kp / kOzTk));
+    ozaki_slice_b_kernel<<<gb, kOzSliceThreads, 0, st>>>(B, ldb, (int)K, (int)N, eb, s, B8, Kp);
     prof_end(ctx, st, kClsOther, 8.0 * (M * K + K * N) + (double)s * Kp * (M + N));  // bytes
     B2M_LAUNCHED(ctx);
     CUtensorMap ma, mb;
