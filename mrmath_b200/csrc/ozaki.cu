@@ -244,11 +244,12 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 // (d = 2 .. s + 1, 64 TMEM columns each, 512 in all) live for the whole K range: per 32-wide
 // k-step the producer (warp 8) loads the s slice tiles of A (128 x 32 bytes) and of B (64 x 32),
 // 32-byte swizzle, into one of four stages; the MMA issuer (one thread of warp 9) runs the
-// s (s + 1) / 2 pairs of the step (one K = 32 MMA each) into the accumulator of d = p + q; the
+// s (s + 1) / 2 pairs of the step, up to four in one MMA, into the accumulators of d = p + q; the
 // epilogue warps drain the accumulators into FP64 once per K chunk (a chunk keeps every S_d an
-// exact int32 sum).  Per k-step the tensor pipe gets s (s + 1) / 2 MMAs for 6 s KiB of operands,
+// exact int32 sum).  Per k-step the tensor pipe gets s (s + 1) / 2 pairs for 6 s KiB of operands,
 // about three times the reuse of the pair-major kernel above, whose slice pairs each reload both
-// tiles.
+// tiles.  Order 8192, s = 8: 16.0 ms with an MMA a pair, bound by the reads of shared memory; 13.3 ms with
+// four pairs an MMA (3.0 POP/s; 15.4 ms when the power cap holds the clock).
 constexpr int KBM = 128, KBN = 64, KBK = 32;
 constexpr int kKmTileA = KBM * KBK, kKmTileB = KBN * KBK;  // 4 KiB, 2 KiB
 constexpr int kKmMaxSlices = 8;
@@ -259,22 +260,25 @@ __device__ __forceinline__ uint64_t sw32_desc(uint32_t saddr) {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(256 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)6 << 61);
 }
-__host__ __device__ constexpr uint32_t i8_idesc_m128n64() {
-    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(KBN >> 3) << 17) | ((uint32_t)(KBM >> 4) << 24);
+// M = 128, N = 64 nb
+__host__ __device__ constexpr uint32_t km_idesc(int nb) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nb * KBN >> 3) << 17) | ((uint32_t)(KBM >> 4) << 24);
 }
 
-// the s (s + 1) / 2 MMAs of one k-step for a compile-time s: descriptors are the stage's base
-// descriptors plus constants, and the first MMA of every accumulator (pa = 1 in this order) of a
-// chunk's first k-step starts it
-template <int S>
-__device__ __forceinline__ void km_issue_step(uint32_t tmem, uint64_t da0, uint64_t db0, uint32_t idesc, bool first) {
+// The s (s + 1) / 2 slice pairs of one k-step.  For one slice of A the B slices pb = 1, 2, .. are
+// neighbours in shared memory and their accumulators d = pa + pb neighbours in TMEM, so up to four pairs
+// are one MMA of N = 256: A's tile is read once for four pairs, and a step reads 120 KB of shared memory
+// instead of 216 (at 128 bytes a cycle 960 cycles instead of 1,730, under the 1,152 of the arithmetic at
+// s = 8).  The MMAs of pa = 1 reach every accumulator, so they start them in a chunk's first k-step.
+__device__ __forceinline__ void km_issue_step(int s, uint32_t tmem, uint64_t da0, uint64_t db0, bool first) {
 #pragma unroll
-    for (int pa = 1; pa <= S; ++pa) {
+    for (int pa = 1; pa <= kKmMaxSlices; ++pa) {
 #pragma unroll
-        for (int pb = 1; pa + pb <= S + 1; ++pb) {
-            const int d = pa + pb;
-            umma_i8(tmem + (uint32_t)((d - 2) * KBN), da0 + (uint64_t)(((pa - 1) * kKmTileA) >> 4),
-                    db0 + (uint64_t)(((pb - 1) * kKmTileB) >> 4), idesc, (first && pa == 1) ? 0u : 1u);
+        for (int b0 = 0; b0 < kKmMaxSlices + 1 - pa; b0 += 4) {
+            const int nb = min(4, s + 1 - pa - b0);
+            if (nb <= 0) continue;
+            umma_i8(tmem + (uint32_t)((pa - 1 + b0) * KBN), da0 + (uint64_t)(((pa - 1) * kKmTileA) >> 4),
+                    db0 + (uint64_t)((b0 * kKmTileB) >> 4), km_idesc(nb), (first && pa == 1) ? 0u : 1u);
         }
     }
 }
@@ -340,34 +344,19 @@ __global__ void __launch_bounds__(kOzThreads, 1)
         }
     } else if (warp == 9) {
         if (lane == 0) {
-            constexpr uint32_t idesc = i8_idesc_m128n64();
             bool ok = true;
             for (int ch = 0; ch < nchunks && ok; ++ch) {
                 const int k0 = ch * p.kchunk, k1 = min(KT, k0 + p.kchunk);
                 // the epilogue must have drained the previous chunk before the accumulators restart
                 if (ch > 0 && !mbar_wait(&acce_bar, (ch - 1) & 1, tmo, 412)) { ok = false; break; }
                 tc_fence_after();
-                uint32_t started = 0u;  // accumulators written in this chunk (bit d - 2)
                 for (int kt = k0; kt < k1; ++kt) {
                     const int st = kt % kKmStages;
                     if (!mbar_wait(&full_bar[st], (kt / kKmStages) & 1, tmo, 413)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem + st * stage_bytes);
                     const uint32_t sb = sa + (uint32_t)(s * kKmTileA);
-                    if (s == kKmMaxSlices) {
-                        km_issue_step<kKmMaxSlices>(tmem, sw32_desc(sa), sw32_desc(sb), idesc, kt == k0);
-                    } else {
-                        for (int pa = 1; pa <= s; ++pa) {
-                            for (int pb = 1; pa + pb <= s + 1; ++pb) {
-                                const int d = pa + pb;
-                                const uint32_t tacc = tmem + (uint32_t)((d - 2) * KBN);
-                                const uint32_t acc = (started >> (d - 2)) & 1u;
-                                umma_i8(tacc, sw32_desc(sa + (uint32_t)((pa - 1) * kKmTileA)),
-                                        sw32_desc(sb + (uint32_t)((pb - 1) * kKmTileB)), idesc, acc);
-                                started |= 1u << (d - 2);
-                            }
-                        }
-                    }
+                    km_issue_step(s, tmem, sw32_desc(sa), sw32_desc(sb), kt == k0);
                     umma_commit(&empty_bar[st]);
                 }
                 umma_commit(&accf_bar);
