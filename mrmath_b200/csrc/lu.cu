@@ -22,6 +22,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "panel.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -428,8 +429,9 @@ __global__ void __launch_bounds__(256, 2) panel_rank_update_kernel(double* A, in
     }
 }
 
-// U12 = L11^-1 A12 for one outer panel in a single launch: L11 unit lower (k <= 256 rows, at L with
-// row stride ldl), the right-hand sides k x ncols at B.  A CTA owns NC columns, held in shared memory
+// U12 = L11^-1 A12 for one outer panel in a single launch, and the diagonal blocks of the solves with many right-hand
+// sides: L11 unit lower or, kUpper, upper (k <= 256 rows, at L with row stride ldl, from the last block up), the
+// right-hand sides k x ncols at B.  A CTA owns NC columns, held in shared memory
 // for the whole solve; per 32-row block of L11 (its block column staged by cp.async, the next one
 // while the current one is used) one warp per 8 columns substitutes the block's triangle, four lanes
 // a column (contributions in ascending order), and all warps subtract the block's contribution from
@@ -443,7 +445,68 @@ constexpr int kTpThreads = 256;
 constexpr int kTpPitch = kTpK + 4;  // columns of X in shared memory (column-major; conflict-free fragments)
 template <int NC> constexpr int tp_smem() { return (NC * kTpPitch + 2 * kTpK * kPanelW) * (int)sizeof(double); }
 
-template <int NC>
+// Back substitution with a block's upper triangle (identity past its rows): lane = column + 8 * (row & 3), x its
+// rows 4 e + (lane >> 3); results to xc.  x / d is the product with the reciprocal corrected by its exact residual
+// (as accurate as the division, whose 144 cycles would be on the chain 32 times); with divisions where a
+// diagonal is far from 1 or a result is not finite.
+__device__ __forceinline__ void tp_upper(const double (*s_t)[kPanelW + 1], int lane, const double (&y)[kPanelW / 4],
+                                         double* xc) {
+    constexpr int kTop = kPanelW / 4 - 1;
+    const int rg = lane >> 3;
+    double dv[kTop + 1], di[kTop + 1];
+    bool odd = false;
+#pragma unroll
+    for (int e = 0; e <= kTop; ++e) {
+        dv[e] = s_t[4 * e + rg][4 * e + rg];
+        di[e] = 1.0 / dv[e];
+        odd = odd || mag_hi(dv[e]) - 0x01700000u >= 0x7d000000u;  // outside 2^-1000 .. 2^1000
+    }
+    auto solve = [&](auto divide) {
+        double x[kTop + 1], d[kTop + 1], r[kTop + 1];
+#pragma unroll
+        for (int e = 0; e <= kTop; ++e) {
+            x[e] = y[e];
+            d[e] = dv[e];
+            r[e] = di[e];
+        }
+        bool finite = true;
+#pragma unroll 1
+        for (int q = kTop; q >= 0; --q) {
+#pragma unroll
+            for (int u = 3; u >= 0; --u) {
+                const double z = x[kTop];
+                double xq;
+                if constexpr (decltype(divide)::value) {
+                    xq = z / d[kTop];
+                } else {
+                    xq = z * r[kTop];
+                    xq = fma(fma(-xq, d[kTop], z), r[kTop], xq);
+                }
+                const double xj = __shfl_sync(0xffffffffu, xq, (lane & 7) + 8 * u);
+                if (rg == u) x[kTop] = xq;
+                const double* uc = &s_t[rg][4 * q + u];
+                if (rg < u) x[kTop] = fma(-uc[4 * q * (kPanelW + 1)], xj, x[kTop]);
+#pragma unroll
+                for (int e = 1; e <= kTop; ++e)
+                    if (q - e >= 0) x[kTop - e] = fma(-uc[4 * (q - e) * (kPanelW + 1)], xj, x[kTop - e]);
+            }
+            finite = finite && mag_hi(x[kTop]) < kInfHi;
+            xc[4 * q + rg] = x[kTop];
+#pragma unroll
+            for (int e = kTop; e > 0; --e) {
+                x[e] = x[e - 1];
+                d[e] = d[e - 1];
+                r[e] = r[e - 1];
+            }
+        }
+        return finite;
+    };
+    bool again = __any_sync(0xffffffffu, odd);
+    if (!again) again = !__all_sync(0xffffffffu, solve(std::false_type{}));
+    if (again) solve(std::true_type{});
+}
+
+template <int NC, bool kUpper>
 __global__ void __launch_bounds__(kTpThreads, 1) trsm_panel_kernel(const double* L, int64_t ldl, double* B,
                                                                    int64_t ldb, int k, int ncols,
                                                                    const int32_t* status) {
@@ -456,36 +519,40 @@ __global__ void __launch_bounds__(kTpThreads, 1) trsm_panel_kernel(const double*
     const int cb = blockIdx.x * NC;
     const int nb = (int)ceil_div(k, kPanelW);
     auto sx = [](int row, int c) { return row * kPanelW + 2 * ((c >> 1) ^ (row & 7)) + (c & 1); };
-    // block column i of L11: rows [32 i, k), columns [32 i, 32 i + 32) -> buffer i & 1 (16-byte pieces)
-    auto stage = [&](int i) {
-        double* dst = s_l + (i & 1) * kTpK * kPanelW;
-        const int r0 = kPanelW * i, c = 2 * (t & 15), col = r0 + c;
+    // block column i of the triangle: columns [32 i, 32 i + 32), rows from 32 i on (kUpper: rows up to and with
+    // the block's) -> buffer `buf` (16-byte pieces)
+    auto stage = [&](int i, int buf) {
+        double* dst = s_l + buf * kTpK * kPanelW;
+        const int r0 = kPanelW * i, c = 2 * (t & 15), col = r0 + c, first = kUpper ? 0 : r0;
+        const int rows = kUpper ? min(k, r0 + kPanelW) : k - r0;
         const int bytes = col + 1 < k ? 16 : (col < k ? 8 : 0);
-        const double* src = L + (int64_t)r0 * ldl + (col < k ? col : 0);
+        const double* src = L + (int64_t)first * ldl + (col < k ? col : 0);
 #pragma unroll 4
-        for (int r = t >> 4; r < k - r0; r += kTpThreads / 16) cp_async16(dst + sx(r, c), src + (int64_t)r * ldl, bytes);
+        for (int r = t >> 4; r < rows; r += kTpThreads / 16) cp_async16(dst + sx(r, c), src + (int64_t)r * ldl, bytes);
         cp_async_commit();
     };
-    stage(0);
+    stage(kUpper ? nb - 1 : 0, 0);
     batched_copy<kTpThreads, 8, double>(t, kTpK * NC,
         [&](int e) {
             const int r = e / NC, c = e % NC;
             return (r < k && cb + c < ncols) ? B[(int64_t)r * ldb + cb + c] : 0.0;
         },
         [&](int e, double v) { s_x[(e % NC) * kTpPitch + e / NC] = v; });
-    for (int i = 0; i < nb; ++i) {
-        if (i + 1 < nb) {
-            stage(i + 1);
+    for (int step = 0; step < nb; ++step) {
+        const int i = kUpper ? nb - 1 - step : step;
+        if (step + 1 < nb) {
+            stage(kUpper ? i - 1 : i + 1, (step + 1) & 1);
             cp_async_wait<1>();
         } else {
             cp_async_wait<0>();
         }
         __syncthreads();
-        const double* lb = s_l + (i & 1) * kTpK * kPanelW;  // lb[sx(r - 32 i, q)] = L[r][32 i + q]
+        const double* lb = s_l + (step & 1) * kTpK * kPanelW;  // lb[sx(r - 32 i, q)] = L[r][32 i + q]; kUpper: lb[sx(r, q)]
         const int r0 = kPanelW * i, bw = min(kPanelW, k - r0);
         for (int e = t; e < kPanelW * kPanelW; e += kTpThreads) {  // the triangle, for constant offsets below
             const int r = e >> 5, c = e & 31;
-            s_t[r][c] = (r < bw && c < r) ? lb[sx(r, c)] : 0.0;
+            if constexpr (kUpper) s_t[r][c] = (c < bw && r <= c) ? lb[sx(r0 + r, c)] : (r == c ? 1.0 : 0.0);
+            else s_t[r][c] = (r < bw && c < r) ? lb[sx(r, c)] : 0.0;
         }
         __syncthreads();
         if (warp < NC / 8) {
@@ -495,9 +562,10 @@ __global__ void __launch_bounds__(kTpThreads, 1) trsm_panel_kernel(const double*
             double x[kPanelW / 4];
 #pragma unroll
             for (int e = 0; e < kPanelW / 4; ++e) x[e] = xc[4 * e + rg];
+            if constexpr (kUpper) tp_upper(s_t, lane, x, xc);
             const double* lt = &s_t[rg][0];
 #pragma unroll 1
-            for (int q = 0; q < kPanelW / 4; ++q, lt += 4 * (kPanelW + 1) + 4) {
+            for (int q = 0; !kUpper && q < kPanelW / 4; ++q, lt += 4 * (kPanelW + 1) + 4) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const double xi = __shfl_sync(0xffffffffu, x[0], (lane & 7) + 8 * u);
@@ -512,13 +580,13 @@ __global__ void __launch_bounds__(kTpThreads, 1) trsm_panel_kernel(const double*
             }
         }
         __syncthreads();
-        // rows below the block (only full blocks have any), 16 x 8 tiles:
+        // rows below the block (only full blocks have any; kUpper: above it), 16 x 8 tiles:
         // a = L[g][k + tq], L[g + 8][k + tq], b = x[k + tq][g], c = rows g, g + 8, columns 2 tq, 2 tq + 1
         const int g = lane >> 2, tq = lane & 3;
-        const int mt = (k - r0 - bw + 15) / 16;
+        const int mt = (kUpper ? r0 : k - r0 - bw + 15) / 16, row0 = kUpper ? 0 : r0;
         for (int tile = warp; tile < mt * (NC / 8); tile += kTpThreads / 32) {
-            const int c8 = 8 * (tile % (NC / 8)), ra = bw + 16 * (tile / (NC / 8)) + g, rb = ra + 8;
-            const bool oka = r0 + ra < k, okb = r0 + rb < k;
+            const int c8 = 8 * (tile % (NC / 8)), ra = (kUpper ? 0 : bw) + 16 * (tile / (NC / 8)) + g, rb = ra + 8;
+            const bool oka = row0 + ra < k, okb = row0 + rb < k;
             double acc[4] = {0.0, 0.0, 0.0, 0.0};
             const double* xb = s_x + (c8 + g) * kTpPitch + r0 + tq;
 #pragma unroll
@@ -530,11 +598,11 @@ __global__ void __launch_bounds__(kTpThreads, 1) trsm_panel_kernel(const double*
                     : "+d"(acc[0]), "+d"(acc[1]), "+d"(acc[2]), "+d"(acc[3])
                     : "d"(a0), "d"(a1), "d"(b0));
             }
-            double* xd = s_x + (c8 + 2 * tq) * kTpPitch + r0;
+            double* xd = s_x + (c8 + 2 * tq) * kTpPitch + row0;
             if (oka) { xd[ra] -= acc[0]; xd[kTpPitch + ra] -= acc[1]; }
             if (okb) { xd[rb] -= acc[2]; xd[kTpPitch + rb] -= acc[3]; }
         }
-        __syncthreads();  // the buffer of block i is restaged for block i + 2
+        __syncthreads();  // the buffer of this step is restaged for the one after the next
     }
     for (int e = t; e < kTpK * NC; e += kTpThreads) {
         const int r = e / NC, c = e % NC;
@@ -854,11 +922,42 @@ struct TriSolve {
     int64_t ldb, bn, bcols, bc0, ncols;
 };
 
+// B (k <= 256 rows, ncols columns) <- T^-1 B in one launch, T unit lower or upper.  8 columns a CTA while
+// the SMs hold them all, then 32.
+int32_t launch_trsm_panel(Ctx* ctx, cudaStream_t st, const double* T, int64_t ldt, double* B, int64_t ldb, int k,
+                          int64_t ncols, bool upper) {
+    const bool few = ncols <= 8 * ctx->num_sms;
+    const auto kern = upper ? (few ? trsm_panel_kernel<8, true> : trsm_panel_kernel<32, true>)
+                            : (few ? trsm_panel_kernel<8, false> : trsm_panel_kernel<32, false>);
+    const int smem = few ? tp_smem<8>() : tp_smem<32>();
+    std::atomic<int>& attr = device_flag((const void*)kern, 0, ctx->device);
+    if (!attr.load()) {
+        B2M_CU(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        attr.store(1);
+    }
+    prof_begin(ctx, st, kClsTrsm);
+    B2M_CU(ctx, launch_k(ctx, kern, dim3((unsigned)ceil_div(ncols, few ? 8 : 32)), dim3(kTpThreads), (size_t)smem, st,
+                         T, ldt, B, ldb, k, (int)ncols, (const int32_t*)ctx->d_status));
+    prof_end(ctx, st, kClsTrsm, 8.0 * (k * (double)k / 2 + 2.0 * k * (double)ncols));  // bytes
+    B2M_LAUNCHED(ctx);
+    return B2M_OK;
+}
+
+// Whether a diagonal block of the recursive solves goes to launch_trsm_panel (which wants 16-byte aligned pairs of
+// the triangle), and where a larger one is split.  Down to 32 rows by recursion, with a
+// product at every level, the inverse of order 512 took 977 us, of order 1500 3.56 ms; with blocks of 256 rows in one
+// launch 680 us and 2.70 ms.
+bool trsm_whole(const TriSolve& t, int64_t k) { return k <= kTpK && (t.lda & 1) == 0 && aligned16(t.A); }
+int64_t trsm_split(int64_t k) { return k > kTpK ? round_up((k + 1) / 2, kTpK) : split_cols(k); }
+
 int32_t trsm_lower_rec(Ctx* ctx, cudaStream_t st, const TriSolve& t, int64_t r0, int64_t br0, int64_t k) {
     if (k <= kPanelW)
         return launch_trsm_small_impl<double>(ctx, st, t.A + r0 * t.lda + r0, t.lda, t.B + br0 * t.ldb + t.bc0, t.ldb,
                                          (int)k, (int)t.ncols, false);
-    const int64_t k1 = split_cols(k), k2 = k - k1;
+    if (trsm_whole(t, k))
+        return launch_trsm_panel(ctx, st, t.A + r0 * t.lda + r0, t.lda, t.B + br0 * t.ldb + t.bc0, t.ldb, (int)k,
+                                 t.ncols, false);
+    const int64_t k1 = trsm_split(k), k2 = k - k1;
     B2M_TRY(trsm_lower_rec(ctx, st, t, r0, br0, k1));
     DOperand a{t.A, t.lda, t.n, t.n, r0 + k1, r0, true};
     DOperand b{t.B, t.ldb, t.bn, t.bcols, br0, t.bc0, false};
@@ -870,7 +969,10 @@ int32_t trsm_upper_rec(Ctx* ctx, cudaStream_t st, const TriSolve& t, int64_t r0,
     if (k <= kPanelW)
         return launch_trsm_small_impl<double>(ctx, st, t.A + r0 * t.lda + r0, t.lda, t.B + br0 * t.ldb + t.bc0, t.ldb,
                                          (int)k, (int)t.ncols, true);
-    const int64_t k1 = split_cols(k), k2 = k - k1;
+    if (trsm_whole(t, k))
+        return launch_trsm_panel(ctx, st, t.A + r0 * t.lda + r0, t.lda, t.B + br0 * t.ldb + t.bc0, t.ldb, (int)k,
+                                 t.ncols, true);
+    const int64_t k1 = trsm_split(k), k2 = k - k1;
     B2M_TRY(trsm_upper_rec(ctx, st, t, r0 + k1, br0 + k1, k2));
     DOperand a{t.A, t.lda, t.n, t.n, r0, r0 + k1, true};
     DOperand b{t.B, t.ldb, t.bn, t.bcols, br0 + k1, t.bc0, false};
@@ -957,14 +1059,6 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
     };
     const int64_t pm_ld = round_up(n, 64);
     PriorityScope hi(ctx, true);  // this stream's launches are the critical path (see launch_k)
-    std::atomic<int>& attr = device_flag((const void*)trsm_panel_kernel<8>, 0, ctx->device);
-    if (!attr.load()) {
-        B2M_CU(ctx, cudaFuncSetAttribute(trsm_panel_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tp_smem<8>()));
-        B2M_CU(ctx, cudaFuncSetAttribute(trsm_panel_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tp_smem<32>()));
-        attr.store(1);
-    }
     for (int64_t k0 = 0; k0 < n; k0 += kOuterNB) {
         const int64_t w = std::min(kOuterNB, n - k0), k1 = k0 + w;
         int32_t* pmap = pmap2 + ((k0 / kOuterNB) & 1) * pm_ld;
@@ -1078,15 +1172,7 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
         }
         if (k1 >= n) break;
         auto update = [&](cudaStream_t qs, int64_t cs, int64_t nc) -> int32_t {
-            prof_begin(ctx, qs, kClsTrsm);
-            const bool few = nc <= 8 * ctx->num_sms;
-            B2M_CU(ctx, launch_k(ctx, few ? trsm_panel_kernel<8> : trsm_panel_kernel<32>,
-                                 dim3((unsigned)ceil_div(nc, few ? 8 : 32)), dim3(kTpThreads),
-                                 (size_t)(few ? tp_smem<8>() : tp_smem<32>()), qs,
-                                 (const double*)(A + k0 * ld + k0), ld, A + k0 * ld + cs, ld, (int)w, (int)nc,
-                                 (const int32_t*)ctx->d_status));
-            prof_end(ctx, qs, kClsTrsm, 8.0 * (w * (double)w / 2 + 2.0 * w * (double)nc));  // bytes
-            B2M_LAUNCHED(ctx);
+            B2M_TRY(launch_trsm_panel(ctx, qs, A + k0 * ld + k0, ld, A + k0 * ld + cs, ld, (int)w, nc, false));
             DOperand a{A, ld, n, n, k1, k0, true};
             DOperand b{A, ld, n, n, k0, cs, false};
             return dgemm_tiled(ctx, qs, a, b, A + k1 * ld + cs, ld, n - k1, nc, w, B2M_DO_SUB, true);
