@@ -331,7 +331,8 @@ B2M_API int32_t b2m_dev_MatrixLinEQSolveAdjoint(b2m_ctx* ctx, const double* LUDe
  * mode 0: FP64 LU with partial pivoting; mode 1: FP32 factorisation + FP64 refinement to
  * backward error <= n_i 2^-53, refactored in FP64 when refinement stalls.  info[i] = 0 (leOk) or
  * 1 (leSingular); iters[i] (may be NULL) = refinement steps in mode 1, -1 when FP64 was needed.
- * The first call with a new plan runs the autotuner (it times the candidate tile shapes). */
+ * The first mode-1 call with a new plan runs the autotuner (it times the candidate tile
+ * shapes); mode 0 has one shape. */
 B2M_API int32_t b2m_BatchLinEQSolve(b2m_ctx* ctx, int64_t count, const int32_t* n, const int32_t* nrhs,
                                     const int64_t* a_off, const int64_t* b_off, const double* A, const double* B,
                                     double* X, int32_t mode, int32_t* info, int32_t* iters);

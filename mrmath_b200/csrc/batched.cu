@@ -43,7 +43,6 @@ namespace {
 constexpr int kBThreads = 256;
 constexpr int kBMaxN = 256;
 constexpr int kBMaxK = 8;
-constexpr int kBMaxPW = 32;
 constexpr int kStrip = 2;  // 16 x 8 tiles per warp step of the trailing update
 
 struct BatchArgs {

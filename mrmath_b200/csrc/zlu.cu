@@ -48,14 +48,6 @@ __device__ __forceinline__ double2 cinv(double2 x) {
     const double r = x.x / x.y, den = x.y + r * x.x;
     return make_double2(r / den, -1.0 / den);
 }
-__device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
-    if (fabs(b.x) >= fabs(b.y)) {
-        const double r = b.y / b.x, den = b.x + b.y * r;
-        return make_double2((a.x + r * a.y) / den, (a.y - r * a.x) / den);
-    }
-    const double r = b.x / b.y, den = b.y + b.x * r;
-    return make_double2((a.x * r + a.y) / den, (a.y * r - a.x) / den);
-}
 // x1 - x2 x3 (CSubMul order)
 __device__ __forceinline__ double2 csub_mul(double2 x1, double2 x2, double2 x3) {
     return make_double2(x1.x - x2.x * x3.x + x2.y * x3.y, x1.y - x2.x * x3.y - x2.y * x3.x);
