@@ -1419,11 +1419,16 @@ int32_t small_solve_f64(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld,
 }
 
 // ------------------------------------------------------------------ host side
-struct BatchPlanCache {
-    std::vector<int32_t> n, k;
-    std::vector<int64_t> a_off, b_off;
-    int64_t count = -1;
-};
+// A plan's key in the autotuner's table, which saved tables hold.  Different plans may share one (offsets fold into
+// each other): it chooses a tile shape, never the data of a call.
+static uint64_t plan_signature(int mode, int64_t count, const int32_t* n, const int32_t* k, const int64_t* a_off,
+                               const int64_t* b_off) {
+    uint64_t sig = 1469598103934665603ull ^ (uint64_t)mode;
+    for (int64_t i = 0; i < count; ++i)
+        sig = (sig ^ (uint64_t)(n[i] * 16 + k[i]) ^ ((uint64_t)a_off[i] << 20) ^ ((uint64_t)b_off[i] << 40)) *
+              1099511628211ull;
+    return sig;
+}
 
 int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn, const int32_t* hk,
                     const int64_t* ha_off, const int64_t* hb_off, const double* A, const double* B, double* X,
@@ -1435,9 +1440,6 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
         if (hk[i] < 1 || hk[i] > kBMaxK) return fail(ctx, B2M_ERR_UNSUPPORTED, "batch: system %lld has %d right-hand sides (1..8)", (long long)i, hk[i]);
     }
     // device copies of the plan: n, k, offsets, order (largest first), queue head
-    std::vector<int32_t> order((size_t)count);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return hn[x] > hn[y]; });
     const size_t bytes_i = (size_t)count * 4, bytes_l = (size_t)count * 8;
     const size_t plan_bytes = 3 * bytes_i + 2 * bytes_l + 256;
     void* pplan;
@@ -1449,29 +1451,35 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
     int64_t* dao = reinterpret_cast<int64_t*>(pp + round_up((int64_t)(3 * bytes_i), 256));
     int64_t* dbo = dao + count;
     int32_t* dctr = reinterpret_cast<int32_t*>(dbo + count);
-    uint64_t sig = 1469598103934665603ull ^ (uint64_t)mode;
-    for (int64_t i = 0; i < count; ++i)
-        sig = (sig ^ (uint64_t)(hn[i] * 16 + hk[i]) ^ ((uint64_t)ha_off[i] << 20) ^ ((uint64_t)hb_off[i] << 40)) *
-              1099511628211ull;
-    const bool same_plan = ctx->batch_plan_sig == sig && ctx->batch_plan_dev == pplan;
-    void* ph = nullptr;
-    if (!same_plan) {
+    BatchPlan& plan = ctx->batch_plan;
+    if (plan.dev != pplan || plan.n.size() != (size_t)count || std::memcmp(plan.n.data(), hn, bytes_i) != 0 ||
+        std::memcmp(plan.k.data(), hk, bytes_i) != 0 || std::memcmp(plan.a_off.data(), ha_off, bytes_l) != 0 ||
+        std::memcmp(plan.b_off.data(), hb_off, bytes_l) != 0) {
+        std::vector<int32_t> order((size_t)count);
+        std::iota(order.begin(), order.end(), 0);
+        std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return hn[x] > hn[y]; });
         // the pinned staging buffer may still feed an earlier asynchronous copy
         B2M_CU(ctx, cudaStreamSynchronize(st));
+        void* ph = nullptr;
         B2M_TRY(pinned_get(ctx, plan_bytes + 256, &ph));
-    }
-    if (!same_plan) {
         char* hp = static_cast<char*>(ph);
         std::memcpy(hp, hn, bytes_i);
         std::memcpy(hp + bytes_i, hk, bytes_i);
         std::memcpy(hp + 2 * bytes_i, order.data(), bytes_i);
         std::memcpy(hp + round_up((int64_t)(3 * bytes_i), 256), ha_off, bytes_l);
         std::memcpy(hp + round_up((int64_t)(3 * bytes_i), 256) + bytes_l, hb_off, bytes_l);
+        plan.dev = nullptr;  // (until the copy is enqueued)
         B2M_CU(ctx, cudaMemcpyAsync(pp, hp, round_up((int64_t)(3 * bytes_i), 256) + 2 * bytes_l,
                                     cudaMemcpyHostToDevice, st));
-        ctx->batch_plan_sig = sig;
-        ctx->batch_plan_dev = pplan;
+        plan.n.assign(hn, hn + count);
+        plan.k.assign(hk, hk + count);
+        plan.a_off.assign(ha_off, ha_off + count);
+        plan.b_off.assign(hb_off, hb_off + count);
+        plan.max_n = hn[order[0]];
+        for (int m = 0; m < 2; ++m) plan.sig[m] = plan_signature(m, count, hn, hk, ha_off, hb_off);
+        plan.dev = pplan;
     }
+    const uint64_t sig = ctx->batch_plan_sig = plan.sig[mode];
 
     int occ_sms = ctx->num_sms;
     BatchArgs a{};
@@ -1519,7 +1527,7 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
         }
         const int64_t grid = std::min<int64_t>(count, (int64_t)ctx->num_sms * kLuCtas);
         void* pscr;
-        const int64_t per = lu_scratch(hn[order[0]]);
+        const int64_t per = lu_scratch(plan.max_n);
         B2M_TRY(ws_get(ctx, kWsMatD, (size_t)(grid * per) * sizeof(double), &pscr));
         BatchArgs b = a;
         b.scratch = static_cast<double*>(pscr);
@@ -1568,7 +1576,8 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
         ctx->batch_tunes[sig] = best;
     }
     if (tune_out) *tune_out = best;
-    const GraphKey key{7 + mode * 10, A, B, X, info, count, (int64_t)sig,
+    // (the launches depend on the plan through its count, its largest order and its tile shape only)
+    const GraphKey key{7 + mode * 10, A, B, X, info, count, (int64_t)plan.max_n,
                        best.big_warps * 1000000 + best.pw_large * 10000 + best.pw_small * 100 + best.group_warps,
                        (int64_t)reinterpret_cast<intptr_t>(iters)};
     return run_graph(ctx, st, key, [&](cudaStream_t q) { return mode == 0 ? launch_lu(q) : launch(best, q); });

@@ -83,6 +83,16 @@ struct BatchTune {
     float ms;         // measured time of the whole batch with this shape
 };
 
+// the batched solve's plan that is on the device (kWsPlan): a host copy of what the caller described it
+// by, compared element by element before the device copy is used again
+struct BatchPlan {
+    std::vector<int32_t> n, k;
+    std::vector<int64_t> a_off, b_off;
+    void* dev = nullptr;  // null: none
+    int32_t max_n = 0;    // its largest order
+    uint64_t sig[2] = {}; // its key in the autotuner's table, by mode
+};
+
 // one progress report, enqueued as a host function behind the panel it reports on
 struct ProgressNote {
     b2m_progress_fn fn;
@@ -132,8 +142,8 @@ struct Ctx {
     void* progress_user = nullptr;
     std::vector<ProgressNote> progress_notes;    // host-function payloads of the current call
     std::map<uint64_t, BatchTune> batch_tunes;  // per batch plan
-    uint64_t batch_plan_sig = 0;                 // plan whose metadata is on the device now
-    void* batch_plan_dev = nullptr;
+    uint64_t batch_plan_sig = 0;                 // table key of the last call's plan
+    BatchPlan batch_plan;
 };
 
 // records a message and returns the status (for `return fail(ctx, ...)`)
