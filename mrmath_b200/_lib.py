@@ -176,7 +176,7 @@ class Context:
         self.check(lib.b2m_set_progress(self.h, C.cast(self._progress, vp) if fn is not None else None, None))
 
     def set_wait_limit(self, polls: int) -> None:
-        """Poll limit of the refinement sweeps' bounded waits (< 0: the built-in limit)."""
+        """Poll limit of the refinement sweeps' and the panel clusters' bounded waits (< 0: the built-in limit)."""
         self.check(lib.b2m_set_wait_limit(self.h, polls))
 
     def kernel_launches(self) -> int:

@@ -108,7 +108,7 @@ struct Ctx {
     int chain_clusters4 = -1; // the same for 4-CTA clusters
     int chain_probe_why = 0;  // why it is unusable: step * 1000 + CUDA error (b2m_ctx_info)
     int dsweep_ctas = -1;     // co-resident CTAs of the FP64 blocked sweep (-1: not queried yet)
-    int64_t wait_limit = -1;  // polls of the refinement sweeps' bounded waits (-1: the built-in limit)
+    int64_t wait_limit = -1;  // polls of the bounded waits that take it (b2m_set_wait_limit; -1: the built-in limit)
     size_t smem_optin = 0;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;

@@ -123,6 +123,8 @@ int32_t lu_determinant(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld, 
 // link (up to 8192 rows): moves_out receives the leaf's interchanges as moves; moves_in not null: the
 // 32 columns left of the panel are the leaf before it, whose interchanges (these moves), triangular
 // solve and update the panel's columns still lack, its top rows 32 rows above P included.
+// (Moves name rows of the panel also after a wait that ran out: those of the columns before it.  After a singular
+// column they are not written, and their readers return on status[kInfo].)
 constexpr int kPanelMoves = 128;  // ints of one moves buffer
 struct PanelLink {
     const int32_t* moves_in = nullptr;

@@ -434,7 +434,7 @@ __device__ __forceinline__ int cand_pieces(int col) { return 1 + (kPBk + 1 - (co
 template <int RPT, bool MULTI>
 __global__ void __launch_bounds__(kPNa, 1)
     panel_kernel(double* P, int64_t ld, int m, int w, int R, int row_base, int col_base, int32_t* ipiv,
-                 int32_t* status, PanelLink link) {
+                 int32_t* status, PanelLink link, uint32_t polls) {
     int C = 1, rank = 0;
     if constexpr (MULTI) {
         C = (int)cg::this_cluster().num_blocks();
@@ -453,6 +453,8 @@ __global__ void __launch_bounds__(kPNa, 1)
     __shared__ __align__(8) uint64_t s_bar[kPSlots], s_rbar;    // a column's candidates; a block's pivot rows
     __shared__ int s_pl[kPW], s_ps[kPW];                        // the pivots: local row, CTA
     __shared__ int s_mv[kPMoves];
+    __shared__ int s_late;    // a wait of the cluster ran out
+    __shared__ PCand s_none;  // no candidate
     // Staging of the previous leaf's L21 rows (s_ll) and of its L11, then U12 (s_lt).  In a cluster it
     // lies in s_rcv: slot 0 may be written by CTAs that are done with their prologue, slots 1 .. 13
     // hold s_ll (no candidate of column 1 is sent before every CTA has sent column 0), the last two
@@ -473,6 +475,8 @@ __global__ void __launch_bounds__(kPNa, 1)
         if (tid == 0) {
             for (int j = 0; j < kPSlots; ++j) mbar_init(&s_bar[j], 1);
             mbar_init(&s_rbar, 1);
+            s_late = 0;
+            s_none.row[0] = 0.0;
             fence_barrier_init();
             for (int j = 0; j < min(kPSlots, w); ++j)
                 mbar_arrive_expect_tx(&s_bar[j], (uint32_t)(C * kPNw * 16 * cand_pieces(j)));
@@ -599,7 +603,8 @@ __global__ void __launch_bounds__(kPNa, 1)
     cp_async_wait<0>();
     __syncthreads();
     if constexpr (MULTI) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-    // the pivot of column j among the published candidates, the same in every warp
+    bool late = false;  // this thread, after select() some thread of its warp, gave up a wait (see panel.cuh)
+    // the pivot of column j among the published candidates, the same in every warp (none for a warp that is late)
     auto select = [&](const int j, int& win) -> const PCand* {
         const int slot = j & (kPSlots - 1);
         if constexpr (MULTI) {
@@ -620,9 +625,14 @@ __global__ void __launch_bounds__(kPNa, 1)
             }
             const uint32_t M = __reduce_max_sync(0xffffffffu, mk);
             const uint32_t bal = __ballot_sync(0xffffffffu, mk == M);
-            const uint32_t bal2 = __ballot_sync(0xffffffffu, mk == M && n > 1);
+            const uint32_t bal2 = __ballot_sync(0xffffffffu, late || (mk == M && n > 1));
             int wl = __ffs(bal) - 1;
             if ((bal & (bal - 1)) || bal2) {
+                late = __any_sync(0xffffffffu, late);
+                if (late) {
+                    win = 0;
+                    return &s_none;
+                }
                 double ba = 0.0;
                 int bp = 0x7fffffff;
 #pragma unroll
@@ -658,72 +668,67 @@ __global__ void __launch_bounds__(kPNa, 1)
             return &s_loc[slot][win];
         }
     };
-    // A bounded wait.  A thread that gives up reports it and goes on without waiting again: it still
-    // takes part in the CTA's barriers, so that no other thread is left at one, and nothing is stored.
-    bool late = false;
     auto wait_bar = [&](uint64_t* bar, const uint32_t phase, const int site) {
-        for (uint32_t it = 0; it < (late ? 1u : kSpinLimit); ++it)
-            if (mbar_try_wait_cluster(bar, phase)) return;
-        if (!late) atomicExch(&status[kTimeout], site);
-        late = true;
+        late = !cluster_wait(bar, phase, polls, &s_late, C, status, site);
     };
     auto wait_col = [&](const int j) { wait_bar(&s_bar[j & (kPSlots - 1)], j / kPSlots, 201); };
-    bool stop = false;
+    bool dead = false;  // this warp met a singular column or is late; the CTA leaves at the next barrier 2
+    bool left = false;  // it has left
     if (warp == kPNw) {
         // ---- scribe warp: records each pivot, and the pivot row's part of U inside its block
         // It also composes the interchanges into moves: lane i holds the position whose content ends in
         // position i (sm), lane e < n_extra a position below the leaf that an interchange reached and
         // the one whose content ends there.
-        int sm = lane, my_pos = -1, my_src = -1, n_extra = 0;
-        bool done = true;
-        for (int j = 0; j < w; ++j) {
-            if constexpr (MULTI) {
-                wait_col(j);
-            } else {
-                asm volatile("bar.sync 1, %0;\n" ::"r"(kPNa) : "memory");
-            }
-            int win;
-            const PCand* b = select(j, win);
-            const double v = lane < kPBk ? b->row[lane] : 0.0;
-            if (!(fabs(b->row[0]) > sing_thresh<double>())) {
-                done = false;
-                break;
-            }
-            if (j == 0 && linked && rank == 0 && !late) {
-                // every CTA has read its rows: U12 of the previous leaf takes its place
-#pragma unroll 8
-                for (int r = 0; r < kPW; ++r)
-                    if (lane < w) P[(int64_t)(r - kPW) * ld + lane] = s_lt[r * kPLtPitch + lane];
-            }
-            {
-                const int q = b->pos, a = __shfl_sync(0xffffffffu, sm, j);
-                int other;
-                if (q < w) {
-                    other = __shfl_sync(0xffffffffu, sm, q);
-                    if (lane == q) sm = a;
+        int sm = lane, my_pos = -1, my_src = -1, n_extra = 0, j = 0;
+        for (int jb = 0; jb < w && !left; jb += kPBk) {
+            for (; j < min(jb + kPBk, w); ++j) {
+                if constexpr (MULTI) {
+                    wait_col(j);
                 } else {
-                    const uint32_t hit = __ballot_sync(0xffffffffu, my_pos == q);
-                    const int e = hit ? __ffs(hit) - 1 : n_extra++;
-                    if (!hit && lane == e) my_pos = my_src = q;
-                    other = __shfl_sync(0xffffffffu, my_src, e);
-                    if (lane == e) my_src = a;
+                    asm volatile("bar.sync 1, %0;\n" ::"r"(kPNa) : "memory");
                 }
-                if (lane == j) sm = other;
+                int win;
+                const PCand* b = select(j, win);
+                const double v = lane < kPBk ? b->row[lane] : 0.0;
+                if (!(fabs(b->row[0]) > sing_thresh<double>())) {
+                    dead = true;
+                    break;
+                }
+                if (j == 0 && linked && rank == 0) {
+                    // every CTA has read its rows: U12 of the previous leaf takes its place
+#pragma unroll 8
+                    for (int r = 0; r < kPW; ++r)
+                        if (lane < w) P[(int64_t)(r - kPW) * ld + lane] = s_lt[r * kPLtPitch + lane];
+                }
+                {
+                    const int q = b->pos, a = __shfl_sync(0xffffffffu, sm, j);
+                    int other;
+                    if (q < w) {
+                        other = __shfl_sync(0xffffffffu, sm, q);
+                        if (lane == q) sm = a;
+                    } else {
+                        const uint32_t hit = __ballot_sync(0xffffffffu, my_pos == q);
+                        const int e = hit ? __ffs(hit) - 1 : n_extra++;
+                        if (!hit && lane == e) my_pos = my_src = q;
+                        other = __shfl_sync(0xffffffffu, my_src, e);
+                        if (lane == e) my_src = a;
+                    }
+                    if (lane == j) sm = other;
+                }
+                if (lane < kPBk && (j & (kPBk - 1)) + lane < kPBk && j + lane < kPW) s_u[j][j + lane] = v;
+                if (lane == 0) {
+                    if (rank == 0) ipiv[col_base + j] = row_base + b->pos;
+                    s_pl[j] = b->lrow;
+                    s_ps[j] = MULTI ? win / kPNw : 0;
+                }
             }
-            if (lane < kPBk && (j & (kPBk - 1)) + lane < kPBk && j + lane < kPW) s_u[j][j + lane] = v;
-            if (lane == 0) {
-                if (rank == 0) ipiv[col_base + j] = row_base + b->pos;
-                s_pl[j] = min((unsigned)b->lrow, (unsigned)R - 1u);  // (in range after a wait that ran out, too)
-                s_ps[j] = MULTI ? win / kPNw : 0;
-            }
-            if ((j & (kPBk - 1)) == kPBk - 1 && j + 1 < w) {
-                asm volatile("bar.sync 2, %0;\n" ::"r"(kPNa) : "memory");
-                asm volatile("bar.sync 2, %0;\n" ::"r"(kPNa) : "memory");
-            } else if (j + 1 == w) {
-                asm volatile("bar.sync 2, %0;\n" ::"r"(kPNa) : "memory");
-            }
+            left = bar_any<kPNa>(2, dead);
+            if (jb + kPBk < w && !left) left = bar_any<kPNa>(2, false);
         }
-        if (done && rank == 0 && link.moves_out) {
+        const bool gave_up = MULTI && left && *reinterpret_cast<volatile int*>(&s_late) != 0;
+        // after a wait that ran out the rest of the leaf interchanges nothing: its readers find valid rows
+        if (gave_up && rank == 0 && lane >= j && lane < w) ipiv[col_base + lane] = row_base + lane;
+        if ((!left || gave_up) && rank == 0 && link.moves_out) {
             link.moves_out[lane] = row_base + sm;
             if (lane == 0) link.moves_out[kPW] = n_extra;
             link.moves_out[kPW + 1 + lane] = row_base + my_pos;
@@ -831,7 +836,7 @@ __global__ void __launch_bounds__(kPNa, 1)
                 const int j = jb + t;
                 if constexpr (MULTI) {
                     wait_col(j);
-                    if (tid == 0 && j + kPSlots < w)
+                    if (tid == 0 && !late && j + kPSlots < w)
                         mbar_arrive_expect_tx(&s_bar[j & (kPSlots - 1)],
                                               (uint32_t)(C * kPNw * 16 * cand_pieces(j + kPSlots)));
                 } else {
@@ -849,8 +854,8 @@ __global__ void __launch_bounds__(kPNa, 1)
                 const int2 pl = *reinterpret_cast<const int2*>(&b->pos);
                 const int p = pl.x, lrow = pl.y;
                 if (!(fabs(u[0]) > sing_thresh<double>())) {
-                    if (rank == 0 && tid == 0) atomicExch(&status[kInfo], 1);
-                    stop = true;
+                    if (rank == 0 && tid == 0 && !late) atomicExch(&status[kInfo], 1);
+                    dead = true;
                     break;
                 }
                 const bool mine = MULTI ? win / kPNw == rank : true;
@@ -867,12 +872,12 @@ __global__ void __launch_bounds__(kPNa, 1)
                 }
                 if (t + 1 < bw) publish(j + 1);
             }
-            if (stop) break;
             // ---- block end: the pivot rows as their owners hold them (multipliers, and the columns
             // right of the block without the block's updates) come together in every CTA
             const int c1 = jb + kPBk;
             if (c1 >= w) break;
-            asm volatile("bar.sync 2, %0;\n" ::"r"(kPNa) : "memory");
+            left = bar_any<kPNa>(2, dead);
+            if (left) break;
             if constexpr (MULTI) {
                 for (int e = tid; e < kPBk * (kPW / 2); e += kPNt) {
                     const int t = e / (kPW / 2), q = e - t * (kPW / 2), c = 2 * q;
@@ -908,7 +913,7 @@ __global__ void __launch_bounds__(kPNa, 1)
 #pragma unroll
                 for (int q = 1; q < kPBk; ++q) s_u[jb + q][c] = x[q];
             }
-            if (MULTI && tid == 0)
+            if (MULTI && tid == 0 && !late)
                 mbar_arrive_expect_tx(&s_rbar, (uint32_t)(min(kPBk, w - c1) * (kPW - c1) * 8));
             double l[RPT][kPBk];
 #pragma unroll
@@ -924,7 +929,8 @@ __global__ void __launch_bounds__(kPNa, 1)
                     l[r][q] = x.x; l[r][q + 1] = x.y;
                     act[r][q] = y.x; act[r][q + 1] = y.y;
                 }
-            asm volatile("bar.sync 2, %0;\n" ::"r"(kPNa) : "memory");
+            left = bar_any<kPNa>(2, late);
+            if (left) break;
 #pragma unroll
             for (int i = 0; i < kPBk; i += 2)
 #pragma unroll
@@ -958,12 +964,12 @@ __global__ void __launch_bounds__(kPNa, 1)
                     if (pos[r] >= 0) *reinterpret_cast<double2*>(S + sx(tid + r * kPNt, c)) = x[r];
             }
         }
-        if (!stop) {
+        if (!left) left = bar_any<kPNa>(2, dead);
+        if (!left) {
             // every row goes to its position: rows below the pivots as they are (multipliers), the
             // pivot rows held here with U right of the diagonal
             int* s_pos = reinterpret_cast<int*>(&s_loc[0][0]);
             static_assert(sizeof(s_loc) >= (size_t)kPNt * RPT * sizeof(int), "positions fit");
-            asm volatile("bar.sync 2, %0;\n" ::"r"(kPNa) : "memory");
 #pragma unroll
             for (int r = 0; r < RPT; ++r) s_pos[tid + r * kPNt] = pos[r];
             asm volatile("bar.sync 3, %0;\n" ::"r"(kPNt) : "memory");
@@ -972,7 +978,7 @@ __global__ void __launch_bounds__(kPNa, 1)
             constexpr int BP = kPW / RS < 4 ? kPW / RS : 4, B = 8;
             const int c = 2 * (tid % LPR);
             auto put = [&](int row, double2 x) {
-                if (late || row >= m) return;
+                if (row >= m) return;
                 double* dst = P + (int64_t)row * ld + c;
                 if (c + 1 < w) *reinterpret_cast<double2*>(dst) = x;
                 else if (c < w) *dst = x.x;
@@ -1008,7 +1014,7 @@ __global__ void __launch_bounds__(kPNa, 1)
             }
         }
     }
-    if constexpr (MULTI) cg::this_cluster().sync();  // no CTA leaves while a push to it may be in flight
+    if constexpr (MULTI) cluster_leave(&s_late);
 }
 
 template <int RPT, bool MULTI>
@@ -1027,7 +1033,7 @@ int32_t launch_panel32(Ctx* ctx, cudaStream_t st, int C, double* P, int64_t ld, 
         attr.store(1);
     }
     return launch_cluster(ctx, st, kern, !MULTI, C, kPNa, smem, m, w, sizeof(double), P, ld, m, w, R, row_base, col_base,
-                          ipiv, ctx->d_status, link);
+                          ipiv, ctx->d_status, link, wait_polls(ctx));
 }
 
 }  // namespace

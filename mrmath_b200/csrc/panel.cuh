@@ -1,6 +1,8 @@
 // panel.cuh -- what the partial-pivoting panels share (panel.cu, zlu.cu, batched.cu).
 #pragma once
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace b2m {
@@ -20,6 +22,45 @@ static __device__ __noinline__ int warp_winner(double a, int pos) {
     const uint32_t mp = __reduce_min_sync(0xffffffffu, top ? (uint32_t)pos : 0xffffffffu);
     return __ffs(__ballot_sync(0xffffffffu, top && (uint32_t)pos == mp)) - 1;
 }
+
+// ---- Bounded waits inside a cluster.  A thread whose wait runs out notes it in every CTA's `late` word; its warp
+// stops working and goes on to its CTA's next common barrier (bar_any, __syncthreads_or), where the whole CTA learns
+// of it and leaves the elimination together: which barriers a thread meets never depends on what it saw alone.
+// A warp that has not given up has seen every candidate so far, so what it records is always a valid interchange.
+
+// waits for a phase of this CTA's barrier, for `polls` polls or until a thread of the cluster has given up; false: in vain
+__device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t phase, uint32_t polls, int* late, int C,
+                                             int32_t* status, int site) {
+    for (uint32_t it = 0; it < polls; ++it) {
+        if (mbar_try_wait_cluster(bar, phase)) return true;
+        if ((it & 255u) == 255u && *reinterpret_cast<volatile int*>(late) != 0) break;
+    }
+    atomicExch(&status[kTimeout], site);
+    for (int d = 0; d < C; ++d)
+        asm volatile("st.shared::cluster.u32 [%0], 1;\n" ::"r"(map_rank(late, d)) : "memory");
+    return false;
+}
+// A cluster kernel's end: no CTA leaves while a push to it may be in flight.  Every push that was waited for has
+// arrived.  After a wait that ran out some may not have, and nothing tells when they do, so every CTA then stays for
+// about 100 us, some two hundred times what a push takes.
+__device__ __forceinline__ void cluster_leave(const int* late) {
+    cooperative_groups::this_cluster().sync();
+    if (*reinterpret_cast<const volatile int*>(late) != 0) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 200000) __nanosleep(200);
+    }
+}
+// named barrier of N threads; whether any of them brought `flag`
+template <int N> __device__ __forceinline__ bool bar_any(int id, bool flag) {
+    uint32_t any;
+    asm volatile(
+        "{ .reg .pred p, q; setp.ne.u32 p, %1, 0; bar.red.or.pred q, %2, %3, p; selp.u32 %0, 1, 0, q; }\n"
+        : "=r"(any)
+        : "r"(flag ? 1u : 0u), "r"(id), "n"(N)
+        : "memory");
+    return any != 0;
+}
+inline uint32_t wait_polls(const Ctx* ctx) { return ctx->wait_limit >= 0 ? (uint32_t)ctx->wait_limit : kSpinLimit; }
 
 // One cluster of C CTAs with the critical path's priority.  plain: a kernel without cluster instructions, on one
 // CTA (one with them needs the cluster attribute on a single CTA, too).
