@@ -113,7 +113,7 @@ __device__ __forceinline__ void st_async_elem(uint32_t raddr, float v, uint32_t 
 template <typename T, int W, int RPT>
 __global__ void __launch_bounds__(kPT, 1)
     panel_push_kernel(T* P, int64_t ld, int m, int w, int R, int row_base, int col_base, int32_t* ipiv,
-                      int32_t* status) {
+                      int32_t* status, uint32_t polls) {
     constexpr int RB = W * (int)sizeof(T);  // row bytes
 
     cg::cluster_group cluster = cg::this_cluster();
@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(kPT, 1)
     __shared__ __align__(8) uint64_t bar[2];
     __shared__ T wabs[2][kPWarps];
     __shared__ int widx[2][kPWarps];
+    __shared__ int s_late;  // a wait of the cluster ran out
 
     if (status[kInfo] != 0) return;  // uniform over the cluster: written before this launch
 
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(kPT, 1)
     if (tid == 0) {
         mbar_init(&bar[0], 1);
         mbar_init(&bar[1], 1);
+        s_late = 0;
         fence_barrier_init();
     }
     // load this CTA's rows (row-major in global, column-major here), 16 loads in flight per thread
@@ -197,6 +199,8 @@ __global__ void __launch_bounds__(kPT, 1)
             if (jb + t < w) S[(jb + t) * RS + tid + k * kPT] = act[k][t];
     };
 
+    bool dead = false;  // this warp met a singular column or gave up a wait; the CTA leaves at its next barrier
+    bool left = false;  // it has left
     // CTA-reduce the candidates of column `col` and push them, with the winner's row and the
     // diagonal row `col`, to every CTA of the cluster (block columns are taken from registers)
     auto publish = [&](const int col, T ma, int mi, const int jb) {
@@ -206,7 +210,8 @@ __global__ void __launch_bounds__(kPT, 1)
         for (int k = 0; k < RPT; ++k)
             if (rowg[k] >= 0 && ((mi >= 0 && rowg[k] == mi) || rowg[k] == col)) store_row(k, jb);
         if (lane == 0) { wabs[par][warp] = ma; widx[par][warp] = mi; }
-        __syncthreads();
+        left = __syncthreads_or(dead);
+        if (left) return;
         T a = lane < kPWarps ? wabs[par][lane] : T(0);
         int i = lane < kPWarps ? widx[par][lane] : -1;
         warp_best(a, i);
@@ -232,31 +237,27 @@ __global__ void __launch_bounds__(kPT, 1)
             if (rowg[k] >= 0 && fabs(act[k][0]) > ma) { ma = fabs(act[k][0]); mi = rowg[k]; }
         publish(0, ma, mi, 0);
     }
-    bool stop = false;
-    int jb = 0;
-    for (; jb < w && !stop; jb += BK) {
+    int done = 0;  // columns whose pivot is recorded
+    for (int jb = 0; jb < w && !dead && !left; jb += BK) {
 #pragma unroll
         for (int t = 0; t < BK; ++t) {
             const int j = jb + t;
             if (j >= w) break;
             const int par = j & 1;
-            bool ok = false;
-            for (uint32_t it = 0; it < kSpinLimit; ++it)
-                if (mbar_try_wait_cluster(&bar[par], (j >> 1) & 1)) { ok = true; break; }
-            if (!ok) {
-                atomicExch(&status[kTimeout], 201);
-                stop = true;
-                break;
-            }
-            if (tid == 0 && j + 2 < w) mbar_arrive_expect_tx(&bar[par], phase_bytes);
+            const bool late = !cluster_wait(&bar[par], (j >> 1) & 1, polls, &s_late, C, status, 201);
+            if (tid == 0 && !late && j + 2 < w) mbar_arrive_expect_tx(&bar[par], phase_bytes);
             // every warp derives the same pivot from the C candidates (lane c reads candidate c)
             T babs = T(0);
             int bidx = -1;
             if (lane < C) unpack_cand(&rcand[par][lane][0], babs, bidx);
+            if (late) {  // above every candidate: the whole warp learns of it
+                babs = static_cast<T>(__longlong_as_double(0x7ff8000000000000ll));
+                bidx = 0x7fffffff;
+            }
             warp_best(babs, bidx);
             if (bidx < 0 || !(babs > sing_thresh<T>())) {
-                if (rank == 0 && tid == 0) atomicExch(&status[kInfo], 1);
-                stop = true;
+                if (rank == 0 && tid == 0 && bidx != 0x7fffffff) atomicExch(&status[kInfo], 1);
+                dead = true;
                 break;
             }
             const int bc = bidx / R;  // the CTA that owns the pivot row sent its row
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(kPT, 1)
             const T* dr = &rdrow[par][0];
             const int p = bidx;
             if (rank == 0 && tid == 0) ipiv[col_base + j] = row_base + p;
+            done = j + 1;
             if (tid < W) ublk[t][tid] = u[tid];
             // the interchanged rows' columns outside the block: written lane-per-column by the
             // warp that owns each row (read only after the next barrier)
@@ -298,11 +300,13 @@ __global__ void __launch_bounds__(kPT, 1)
             if (j + 1 >= w) continue;
             if (t + 1 < BK) {
                 publish(j + 1, mb, mbi, jb);
+                if (left) break;
                 continue;
             }
             // ---- block end: correct the block's pivot rows beyond the block (L11^{-1} U12), store
             // the block columns, rank-BK update of the columns to the right, load the next block
-            __syncthreads();
+            left = __syncthreads_or(false);
+            if (left) break;
             for (int c = jb + BK + tid; c < w; c += kPT) {
 #pragma unroll
                 for (int t1 = 1; t1 < BK; ++t1) {
@@ -339,7 +343,11 @@ __global__ void __launch_bounds__(kPT, 1)
             publish(j + 1, ma, mi, jb + BK);
         }
     }
-    if (!stop) {
+    if (!left) left = __syncthreads_or(dead);
+    // (after a wait that ran out the rest of the leaf interchanges nothing: its readers find valid rows)
+    if (left && rank == 0 && tid == 0 && *reinterpret_cast<volatile int*>(&s_late) != 0)
+        for (int j = done; j < w; ++j) ipiv[col_base + j] = row_base + j;
+    if (!left) {
         // the last block's columns are still in registers
         const int jl = ((w - 1) / BK) * BK;
 #pragma unroll
@@ -347,13 +355,13 @@ __global__ void __launch_bounds__(kPT, 1)
             if (rowg[k] >= 0) store_row(k, jl);
     }
     __syncthreads();
-    if (!stop) {
+    if (!left) {
         for (int e = tid; e < nr * w; e += kPT) {
             const int rl = e / w, c = e - rl * w;
             P[(int64_t)(lo + rl) * ld + c] = S[c * RS + rl];
         }
     }
-    cluster.sync();  // no CTA leaves while a push to it may still be in flight
+    cluster_leave(&s_late);
 }
 
 template <typename T, int W, int RPT>
@@ -368,7 +376,7 @@ int32_t launch_push(Ctx* ctx, cudaStream_t st, int C, int R, T* P, int64_t ld, i
         attr.store(1);
     }
     return launch_cluster(ctx, st, kern, false, C, kPT, smem, m, w, sizeof(T), P, ld, m, w, R, row_base, col_base, ipiv,
-                          ctx->d_status);
+                          ctx->d_status, wait_polls(ctx));
 }
 
 

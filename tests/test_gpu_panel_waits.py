@@ -38,3 +38,25 @@ def test_linked_leaves(n, graphs):
         _ends(c, call, lambda x, y: np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1]))
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n", [8200, 16400])  # leaves of 16 and 8 columns
+def test_tall_panels(n):
+    import torch
+    c = _lib.Context()
+    try:
+        g = torch.Generator(device="cuda").manual_seed(n)
+        a = 2.0 * torch.rand((n, n), generator=g, device="cuda", dtype=torch.float64) - 1.0
+
+        def call():
+            lu, idx = a.clone(), torch.zeros(n, dtype=torch.int32, device="cuda")
+            st = torch.zeros(1, dtype=torch.int32, device="cuda")
+            L.dev_MatrixLUDecompInPlace(lu, idx, st, ctx=c)
+            torch.cuda.synchronize()
+            if int(st.item()) != 0:
+                raise _lib.B2MError(int(st.item()), "")
+            return lu, idx
+
+        _ends(c, call, lambda x, y: torch.equal(x[0], y[0]) and torch.equal(x[1], y[1]))
+    finally:
+        c.close()
