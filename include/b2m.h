@@ -112,7 +112,7 @@ B2M_API int32_t     b2m_dev_ReadMatrixFile(b2m_ctx* ctx, const char* path, b2m_m
 B2M_API int32_t     b2m_WriteMatrixFile(const char* path, const double* src, int64_t LineWidth, int64_t width,
                                         int64_t height);
 /* Number of polls after which a bounded wait of the mixed solve's refinement sweeps, or of the thread-block
- * clusters that factor the FP64 LU's panels, gives up
+ * clusters that factor the FP64 and complex LU's panels, gives up
  * (polls < 0 restores the built-in limit, about a second of spinning).  No counterpart in the
  * reference: a lower limit exists to exercise the timeout path -- with 0 polls every dependent
  * wait gives up at once, the call returns B2M_ERR_TIMEOUT and the context stays usable. */

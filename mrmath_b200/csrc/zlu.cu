@@ -224,7 +224,8 @@ __device__ __forceinline__ double2 cinv_lane(double2 v, bool any) {
 
 template <int RPT, bool MULTI>
 __global__ void __launch_bounds__(kZNt, 1)
-    zpanel_kernel(Planes P, int m, int w, int R, int row_base, int32_t* ipiv, int32_t* map, int32_t* status) {
+    zpanel_kernel(Planes P, int m, int w, int R, int row_base, int32_t* ipiv, int32_t* map, int32_t* status,
+                  uint32_t polls) {
     int C = 1, rank = 0;
     if constexpr (MULTI) {
         C = (int)cg::this_cluster().num_blocks();
@@ -232,11 +233,13 @@ __global__ void __launch_bounds__(kZNt, 1)
     }
     extern __shared__ __align__(16) double2 Z[];  // this CTA's rows [R][32], elements swizzled by row
     auto sx = [](int row, int c) -> int { return row * kZLeaf + (c ^ (row & 7)); };
-    __shared__ ZCand s_loc[2][kZNw], s_rcv[2][kZNw * kZMaxC];
+    constexpr int kNone = kZNw * kZMaxC;  // (no candidate: mag 0)
+    __shared__ ZCand s_loc[2][kZNw], s_rcv[2][kNone + 1];
     __shared__ __align__(16) double2 s_u[kZLeaf][kZLeaf], s_l[kZBk][kZBk];
     __shared__ __align__(16) uint32_t s_key[2][kZNw];  // leading words of a lone CTA's candidates
     __shared__ __align__(8) uint64_t s_bar[2], s_rbar;
     __shared__ int s_pl[kZLeaf], s_ps[kZLeaf];
+    __shared__ int s_late;  // a wait of the cluster ran out
     if (status[kInfo] != 0) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int lo = rank * R, nr = max(0, min(m, lo + R) - lo);
@@ -244,6 +247,8 @@ __global__ void __launch_bounds__(kZNt, 1)
         mbar_init(&s_bar[0], 1);
         mbar_init(&s_bar[1], 1);
         mbar_init(&s_rbar, 1);
+        s_late = 0;
+        s_rcv[0][kNone].mag = s_rcv[1][kNone].mag = 0.0;
         fence_barrier_init();
         for (int j = 0; j < min(2, w); ++j)
             mbar_arrive_expect_tx(&s_bar[j], (uint32_t)(C * kZNw * 16 * zcand_pieces(j)));
@@ -262,7 +267,8 @@ __global__ void __launch_bounds__(kZNt, 1)
     cp_async_wait<0>();
     __syncthreads();
     if constexpr (MULTI) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-    // the pivot of a column among the cluster's candidates, the same in every warp
+    bool late = false;  // this thread, after select() some thread of its warp, gave up a wait (see panel.cuh)
+    // the pivot of a column among the cluster's candidates, the same in every warp (kNone for a warp that is late)
     auto select = [&](const ZCand* cands) -> int {
         if constexpr (!MULTI) {
             const uint4 kv = *reinterpret_cast<const uint4*>(&s_key[cands == s_rcv[1] ? 1 : 0][0]);
@@ -288,9 +294,11 @@ __global__ void __launch_bounds__(kZNt, 1)
         int q = k[0] == mk ? lane : lane + 32;
         const uint32_t M = __reduce_max_sync(0xffffffffu, mk);
         const uint32_t bal = __ballot_sync(0xffffffffu, mk == M);
-        const uint32_t bal2 = __ballot_sync(0xffffffffu, mk == M && k[0] == k[1]);
+        const uint32_t bal2 = __ballot_sync(0xffffffffu, late || (mk == M && k[0] == k[1]));
         int wl = __ffs(bal) - 1;
         if ((bal & (bal - 1)) || bal2) {
+            late = __any_sync(0xffffffffu, late);
+            if (late) return kNone;
             double ba = 0.0;
             int bp = 0x7fffffff;
 #pragma unroll
@@ -306,14 +314,8 @@ __global__ void __launch_bounds__(kZNt, 1)
         const int win = wl + (((odd >> wl) & 1u) ? 32 : 0);
         return win < cnt ? win : 0;
     };
-    // A bounded wait.  A thread that gives up reports it and goes on without waiting again: it still
-    // takes part in the CTA's barriers, and nothing is stored.
-    bool late = false;
     auto wait_bar = [&](uint64_t* bar, const uint32_t phase, const int site) {
-        for (uint32_t it = 0; it < (late ? 1u : kSpinLimit); ++it)
-            if (mbar_try_wait_cluster(bar, phase)) return;
-        if (!late) atomicExch(&status[kTimeout], site);
-        late = true;
+        late = !cluster_wait(bar, phase, polls, &s_late, C, status, site);
     };
     int pos[RPT];
     double2 act[RPT][kZBk];
@@ -397,7 +399,8 @@ __global__ void __launch_bounds__(kZNt, 1)
                     st_async16(push_dst + slot * (uint32_t)sizeof(s_rcv[0]) + 16 * q, src[q], push_bar + 8 * slot);
         }
     };
-    bool stop = false;
+    bool dead = false;  // this warp met a singular column or is late; the CTA leaves at its next common barrier
+    bool left = false;  // it has left
     publish(0);
     for (int jb = 0; jb < w; jb += kZBk) {
         const int bw = min(kZBk, w - jb);
@@ -406,7 +409,7 @@ __global__ void __launch_bounds__(kZNt, 1)
             const int j = jb + t;
             if constexpr (MULTI) wait_bar(&s_bar[j & 1], (j >> 1) & 1, 204);
             else __syncthreads();
-            if (MULTI && tid == 0 && j + 2 < w)
+            if (MULTI && tid == 0 && !late && j + 2 < w)
                 mbar_arrive_expect_tx(&s_bar[j & 1], (uint32_t)(C * kZNw * 16 * zcand_pieces(j + 2)));
             const int win = select(s_rcv[j & 1]);
             const ZCand& b = s_rcv[j & 1][win];
@@ -416,8 +419,8 @@ __global__ void __launch_bounds__(kZNt, 1)
             const double2 rinv = b.rinv;
             const int2 pl = *reinterpret_cast<const int2*>(&b.pos);
             if (!(b.mag > 10.0 / DBL_MAX)) {
-                if (rank == 0 && tid == 0) atomicExch(&status[kInfo], 1);
-                stop = true;
+                if (rank == 0 && tid == 0 && !late) atomicExch(&status[kInfo], 1);
+                dead = true;
                 break;
             }
             const bool mine = MULTI ? win / kZNw == rank : true;
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(kZNt, 1)
                 if (lane < kZBk - t && j + lane < kZLeaf) s_u[j][j + lane] = b.row[lane];
                 if (lane == 0) {
                     if (rank == 0) ipiv[row_base + j] = row_base + pl.x;
-                    s_pl[j] = min((unsigned)pl.y, (unsigned)R - 1u);  // (in range after a wait that ran out, too)
+                    s_pl[j] = pl.y;
                     s_ps[j] = MULTI ? win / kZNw : 0;
                 }
             }
@@ -444,12 +447,12 @@ __global__ void __launch_bounds__(kZNt, 1)
             }
             if (t + 1 < bw) publish(j + 1);
         }
-        if (stop) break;
         // ---- block end: the pivot rows as their owners hold them (multipliers, and the columns right
         // of the block without the block's updates) come together in every CTA
         const int c1 = jb + kZBk;
         if (c1 >= w) break;
-        __syncthreads();
+        left = __syncthreads_or(dead);
+        if (left) break;
         for (int e = tid; e < kZBk * kZLeaf; e += kZNt) {
             const int t = e / kZLeaf, c = e % kZLeaf;
             if (s_ps[jb + t] == rank && c >= jb) {
@@ -476,8 +479,9 @@ __global__ void __launch_bounds__(kZNt, 1)
 #pragma unroll
             for (int q = 1; q < kZBk; ++q) s_u[jb + q][c] = x[q];
         }
-        if (MULTI && tid == 0) mbar_arrive_expect_tx(&s_rbar, (uint32_t)(kZBk * (kZLeaf - c1) * 16));
-        __syncthreads();
+        if (MULTI && tid == 0 && !late) mbar_arrive_expect_tx(&s_rbar, (uint32_t)(kZBk * (kZLeaf - c1) * 16));
+        left = __syncthreads_or(late);
+        if (left) break;
 #pragma unroll 1
         for (int c = c1; c < kZLeaf; c += 4) {  // four columns a step; the first eight stay in registers
             double2 x[RPT][4];
@@ -514,8 +518,8 @@ __global__ void __launch_bounds__(kZNt, 1)
             }
         }
     }
-    __syncthreads();
-    if (!stop) {
+    if (!left) left = __syncthreads_or(dead);
+    if (!left) {
         // every row goes to its position: rows below the pivots as they are (multipliers), the pivot
         // rows held here with U from the diagonal on
         int* s_pos = reinterpret_cast<int*>(&s_loc[0][0]);
@@ -535,7 +539,7 @@ __global__ void __launch_bounds__(kZNt, 1)
             }
 #pragma unroll
             for (int q = 0; q < B; ++q) {
-                const bool ok = !late && fin[q] < m && r0 + q * kZNw < nr;
+                const bool ok = fin[q] < m && r0 + q * kZNw < nr;
                 double* dr = P.re + (int64_t)fin[q] * P.ld + lane;
                 double* di = P.im + (int64_t)fin[q] * P.ld + lane;
                 if (ok && lane < w) *dr = v[q].x;
@@ -544,7 +548,7 @@ __global__ void __launch_bounds__(kZNt, 1)
             }
         }
     }
-    if constexpr (MULTI) cg::this_cluster().sync();  // no CTA leaves while a push to it may be in flight
+    if constexpr (MULTI) cluster_leave(&s_late);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -896,7 +900,7 @@ int32_t launch_zpanel(Ctx* ctx, cudaStream_t st, const Planes& P, int m, int w, 
         attr.store(1);
     }
     return launch_cluster(ctx, st, kern, !MULTI, C, kZNt, (size_t)R * kZLeaf * sizeof(double2), m, w, sizeof(double2), P, m, w,
-                          R, row_base, ipiv, map, ctx->d_status);
+                          R, row_base, ipiv, map, ctx->d_status, wait_polls(ctx));
 }
 
 // factor columns [c0, c0 + width), rows [c0, n); interchanges apply to all of [0, n)

@@ -60,3 +60,21 @@ def test_tall_panels(n):
         _ends(c, call, lambda x, y: torch.equal(x[0], y[0]) and torch.equal(x[1], y[1]))
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("n", [300, 600, 1300])
+def test_complex_panels(n):
+    c = _lib.Context()
+    try:
+        r = inputs.rng(n)
+        a = (r.random_sample((n, n)) - 0.5) + 1j * (r.random_sample((n, n)) - 0.5)
+
+        def call():
+            lu = a.copy()
+            st, idx = L.CplxMatrixLUDecompInPlace(lu, ctx=c)
+            assert st == 0
+            return lu, idx
+
+        _ends(c, call, lambda x, y: np.array_equal(x[0], y[0]) and np.array_equal(x[1], y[1]))
+    finally:
+        c.close()
