@@ -982,7 +982,8 @@ __device__ __forceinline__ void lu_upper(LuSlice<NW, W>& s, int t, int bar, cons
         if (warp == 0) {
             // lane = right-hand side + 8 * (row & 3); rows from the last one up, four a step.  x / d is
             // the product with the reciprocal corrected by its exact residual; where a diagonal is far
-            // from 1 or a result is not finite, the block is solved again with divisions.
+            // from 1 the block, and where a result is not finite its right-hand side, is solved with
+            // divisions.  So a right-hand side's result does not depend on its neighbours.
             const int q = lane & 7, rg = lane >> 3;
             double dv[W / 4], di[W / 4];
             bool odd = false;
@@ -995,7 +996,7 @@ __device__ __forceinline__ void lu_upper(LuSlice<NW, W>& s, int t, int bar, cons
             double y0[W / 4];
 #pragma unroll
             for (int i = 0; i < W / 4; ++i) y0[i] = 4 * i + rg < bs ? y[(b0 + 4 * i + rg) * kBMaxK + q] : 0.0;
-            auto solve = [&](auto divide) {
+            auto solve = [&](auto divide, bool put) {
                 constexpr bool kDivide = decltype(divide)::value;
                 constexpr int kTop = W / 4 - 1;
                 double x[W / 4], d[W / 4], r[W / 4];
@@ -1027,7 +1028,7 @@ __device__ __forceinline__ void lu_upper(LuSlice<NW, W>& s, int t, int bar, cons
                             if (i4 - i >= 0) x[kTop - i] = fma(-uc[4 * (i4 - i)], xj, x[kTop - i]);
                     }
                     finite = finite && mag_hi(x[kTop]) < kInfHi;
-                    if (4 * i4 + rg < bs) y[(b0 + 4 * i4 + rg) * kBMaxK + q] = x[kTop];
+                    if (put && 4 * i4 + rg < bs) y[(b0 + 4 * i4 + rg) * kBMaxK + q] = x[kTop];
 #pragma unroll
                     for (int i = kTop; i > 0; --i) {
                         x[i] = x[i - 1];
@@ -1037,9 +1038,9 @@ __device__ __forceinline__ void lu_upper(LuSlice<NW, W>& s, int t, int bar, cons
                 }
                 return finite;
             };
-            bool again = __any_sync(0xffffffffu, odd);
-            if (!again) again = !__all_sync(0xffffffffu, solve(std::false_type{}));
-            if (again) solve(std::true_type{});
+            uint32_t again = __any_sync(0xffffffffu, odd) ? 0xffffffffu : 0u;
+            if (!again) again = __ballot_sync(0xffffffffu, !solve(std::false_type{}, true));
+            if (again) solve(std::true_type{}, (again & (0x01010101u << q)) != 0);
         }
         lu_sync<NW>(bar);
         // fold the block into the rows above (only full blocks of 4 k: bs < W only in the last one)

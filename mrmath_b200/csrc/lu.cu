@@ -448,7 +448,8 @@ template <int NC> constexpr int tp_smem() { return (NC * kTpPitch + 2 * kTpK * k
 // Back substitution with a block's upper triangle (identity past its rows): lane = column + 8 * (row & 3), x its
 // rows 4 e + (lane >> 3); results to xc.  x / d is the product with the reciprocal corrected by its exact residual
 // (as accurate as the division, whose 144 cycles would be on the chain 32 times); with divisions where a
-// diagonal is far from 1 or a result is not finite.
+// diagonal is far from 1, and in the columns with a result that is not finite.  So a column's result does not
+// depend on its neighbours.
 __device__ __forceinline__ void tp_upper(const double (*s_t)[kPanelW + 1], int lane, const double (&y)[kPanelW / 4],
                                          double* xc) {
     constexpr int kTop = kPanelW / 4 - 1;
@@ -461,7 +462,7 @@ __device__ __forceinline__ void tp_upper(const double (*s_t)[kPanelW + 1], int l
         di[e] = 1.0 / dv[e];
         odd = odd || mag_hi(dv[e]) - 0x01700000u >= 0x7d000000u;  // outside 2^-1000 .. 2^1000
     }
-    auto solve = [&](auto divide) {
+    auto solve = [&](auto divide, bool put) {
         double x[kTop + 1], d[kTop + 1], r[kTop + 1];
 #pragma unroll
         for (int e = 0; e <= kTop; ++e) {
@@ -491,7 +492,7 @@ __device__ __forceinline__ void tp_upper(const double (*s_t)[kPanelW + 1], int l
                     if (q - e >= 0) x[kTop - e] = fma(-uc[4 * (q - e) * (kPanelW + 1)], xj, x[kTop - e]);
             }
             finite = finite && mag_hi(x[kTop]) < kInfHi;
-            xc[4 * q + rg] = x[kTop];
+            if (put) xc[4 * q + rg] = x[kTop];
 #pragma unroll
             for (int e = kTop; e > 0; --e) {
                 x[e] = x[e - 1];
@@ -501,9 +502,9 @@ __device__ __forceinline__ void tp_upper(const double (*s_t)[kPanelW + 1], int l
         }
         return finite;
     };
-    bool again = __any_sync(0xffffffffu, odd);
-    if (!again) again = !__all_sync(0xffffffffu, solve(std::false_type{}));
-    if (again) solve(std::true_type{});
+    uint32_t again = __any_sync(0xffffffffu, odd) ? 0xffffffffu : 0u;
+    if (!again) again = __ballot_sync(0xffffffffu, !solve(std::false_type{}, true));
+    if (again) solve(std::true_type{}, (again & (0x01010101u << (lane & 7))) != 0);
 }
 
 template <int NC, bool kUpper>
