@@ -825,20 +825,25 @@ __global__ void __launch_bounds__(kPermThreads) perm_from_ipiv_kernel(const int3
     }
 }
 
-// the same for larger orders, step by step in global memory
-__global__ void perm_from_ipiv_serial_kernel(const int32_t* ipiv, int n, int32_t* perm) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = i;
+// the same for larger orders, step by step: on a copy in shared memory while n ints fit there, else in global memory
+__global__ void perm_from_ipiv_serial_kernel(const int32_t* ipiv, int n, int32_t* perm, int in_smem) {
+    extern __shared__ int32_t ps_dyn[];
+    int32_t* pv = in_smem ? ps_dyn : perm;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) pv[i] = i;
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int i = 0; i < n; ++i) {
             const int q = ipiv[i];
             if (q != i && q >= 0 && q < n) {
-                const int t = perm[i];
-                perm[i] = perm[q];
-                perm[q] = t;
+                const int t = pv[i];
+                pv[i] = pv[q];
+                pv[q] = t;
             }
         }
     }
+    __syncthreads();
+    if (in_smem)
+        for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = pv[i];
 }
 
 // det = (-1)^{#i: ipiv[i] != i} * U[0][0] * U[1][1] * ... in this order (MatrixDeterminant :467-476);
@@ -1326,7 +1331,15 @@ int32_t perm_from_ipiv(Ctx* ctx, cudaStream_t st, const int32_t* ipiv, int64_t n
         }
         perm_from_ipiv_kernel<<<1, kPermThreads, smem, st>>>(ipiv, (int)n, perm);
     } else {
-        perm_from_ipiv_serial_kernel<<<1, 1024, 0, st>>>(ipiv, (int)n, perm);
+        const size_t copy = (size_t)n * sizeof(int32_t);
+        const bool in_smem = copy <= ctx->smem_optin;
+        std::atomic<int>& set = device_flag((const void*)perm_from_ipiv_serial_kernel, 0, ctx->device);
+        if (in_smem && !set.load()) {
+            B2M_CU(ctx, cudaFuncSetAttribute(perm_from_ipiv_serial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)ctx->smem_optin));
+            set.store(1);
+        }
+        perm_from_ipiv_serial_kernel<<<1, 1024, in_smem ? copy : 0, st>>>(ipiv, (int)n, perm, in_smem ? 1 : 0);
     }
     B2M_LAUNCHED(ctx);
     return B2M_OK;
