@@ -69,9 +69,10 @@ B2M_API int32_t     b2m_synchronize(b2m_ctx* ctx);
 /* Progress callback of the LU-based routines, the counterpart of TLinEquProgress
  * (MatrixConst.pas:31, called with numCalc*100 div numCols at LinAlgLU.pas:272-276): `fn(percent,
  * user)` runs on a CUDA host thread after every factored panel of the FP64 LU (every 32, 16 or 8
- * columns), with percent = columns factored * 100 div n, in order.  It must not call CUDA or this
- * library.  While a callback is set, factorisations run without graph replay and a call first
- * waits for the context's previous work.  NULL removes it. */
+ * columns), with percent = columns factored * 100 div n, in order; up to order 256, where the
+ * factorisation is one kernel, the reports follow it together.  The results are those of a call
+ * without reports.  It must not call CUDA or this library.  While a callback is set, factorisations
+ * run without graph replay and a call first waits for the context's previous work.  NULL removes it. */
 typedef void (*b2m_progress_fn)(int32_t percent, void* user);
 B2M_API int32_t     b2m_set_progress(b2m_ctx* ctx, b2m_progress_fn fn, void* user);
 /* ------------------------------------------------------------------ resident matrices

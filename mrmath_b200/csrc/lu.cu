@@ -886,6 +886,14 @@ void CUDART_CB progress_trampoline(void* p) {
     if (note->fn) note->fn(note->percent, note->user);
 }
 
+// TLinEquProgress, queued behind the work on `st`: columns factored * 100 div n
+int32_t report_progress(Ctx* ctx, cudaStream_t st, int64_t columns, int64_t n) {
+    if (!ctx->progress || ctx->progress_notes.size() >= ctx->progress_notes.capacity()) return B2M_OK;
+    ctx->progress_notes.push_back(ProgressNote{ctx->progress, ctx->progress_user, (int32_t)(columns * 100 / n)});
+    B2M_CU(ctx, cudaLaunchHostFunc(st, progress_trampoline, &ctx->progress_notes.back()));
+    return B2M_OK;
+}
+
 // the leaf's interchanges on columns [col_lo, col_hi) (which contain the leaf's own columns)
 template <typename T>
 int32_t launch_swaps_range(Ctx* ctx, cudaStream_t st, T* A, int64_t ld, int col_lo, int col_hi, int c0, int w,
@@ -1001,12 +1009,6 @@ int32_t lu_rec(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t n, int6
                                      ipiv));
         B2M_TRY(launch_swaps_range<double>(ctx, st, A, ld, (int)sc.col_lo, (int)sc.col_hi, (int)c0, (int)width, ipiv,
                                            perm, sc.pmap));
-        if (ctx->progress && ctx->progress_notes.size() < ctx->progress_notes.capacity()) {
-            // TLinEquProgress: columns factored * 100 div n, queued behind this panel
-            ctx->progress_notes.push_back(
-                ProgressNote{ctx->progress, ctx->progress_user, (int32_t)((c0 + width) * 100 / n)});
-            B2M_CU(ctx, cudaLaunchHostFunc(st, progress_trampoline, &ctx->progress_notes.back()));
-        }
         return B2M_OK;
     }
     // splits on multiples of 16 above the leaf level keep the Schur GEMMs' K on whole TMA k-tiles
@@ -1028,7 +1030,7 @@ int32_t lu_rec(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t n, int6
 constexpr int64_t kOuterNB = 256;  // outer panel width of the blocked FP64 LU
 static_assert(kOuterNB == kTpK, "the panel triangular solve holds one outer panel's rows");
 
-// Blocked right-looking LU with look-ahead (orders n > 2 kOuterNB).  Per outer panel of 256
+// Blocked right-looking LU with look-ahead (orders n > kSmallLu).  Per outer panel of 256
 // columns: (1) the panel is factored right-looking by leaves, each leaf's interchanges kept inside
 // the panel (and recorded in the row map pmap), its U12 formed by the same launch and its rank-w
 // update applied to the rest of the panel (leaf_swap_u12_kernel, panel_rank_update_kernel); (2) the
@@ -1147,11 +1149,7 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
                 B2M_CU(ctx, cudaEventRecord(ctx->ev_leaf_side, ql));
                 leaf_busy = true;
             }
-            if (ctx->progress && ctx->progress_notes.size() < ctx->progress_notes.capacity()) {
-                ctx->progress_notes.push_back(
-                    ProgressNote{ctx->progress, ctx->progress_user, (int32_t)((c0 + wl) * 100 / n)});
-                B2M_CU(ctx, cudaLaunchHostFunc(q, progress_trampoline, &ctx->progress_notes.back()));
-            }
+            B2M_TRY(report_progress(ctx, q, c0 + wl, n));
         }
         if (leaf_busy) B2M_CU(ctx, cudaStreamWaitEvent(q, ctx->ev_leaf_side, 0));
         if (part == 0) return B2M_OK;
@@ -1262,10 +1260,10 @@ int32_t lu_factor_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t 
     //     256: 350 / 429 and about 375 by the blocked driver);
     //   * above, the blocked look-ahead driver with linked leaves (257: 377 / 491, 512: 658 / 931);
     //   * the plain recursion where no workspace or side stream may be used (the allocation-free entry
-    //     point, n <= 512), and up to order 512 with progress reports, which it makes leaf by leaf.
+    //     point, n <= 512).
     // Every order asks for the small orders' scratch and the side streams, so that after a call of any order
     // a smaller one allocates nothing (and can be captured).
-    const bool plain = ctx->fixed_scratch || (ctx->progress && n <= 2 * kOuterNB);
+    const bool plain = ctx->fixed_scratch;
     const bool blocked = !plain && n > kSmallLu;
     void* scratch = nullptr;
     if (!ctx->fixed_scratch) {
@@ -1273,7 +1271,12 @@ int32_t lu_factor_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t 
         B2M_TRY(ws_get(ctx, kWsPmap, std::max(maps, small_lu_scratch(kSmallLu)), &scratch));
         B2M_TRY(ensure_side_stream(ctx));
     }
-    if (!plain && !blocked) return small_lu_f64(ctx, st, A, ld, n, static_cast<double*>(scratch), ipiv, perm);
+    if (!plain && !blocked) {
+        B2M_TRY(small_lu_f64(ctx, st, A, ld, n, static_cast<double*>(scratch), ipiv, perm));
+        for (int64_t c = 0; ctx->progress && c < n; c += leaf)
+            B2M_TRY(report_progress(ctx, st, std::min(n, c + leaf), n));
+        return B2M_OK;
+    }
     int32_t* pmap2 = static_cast<int32_t*>(scratch);
     const GraphKey key{1, A, ipiv, perm, ctx->d_status, ld, n, 0, 0};
     const GraphKey key1{1, A, ipiv, perm, ctx->d_status, ld, n, 0, 1};
