@@ -351,7 +351,8 @@ B2M_API int32_t b2m_dev_BatchLinEQSolve(b2m_ctx* ctx, int64_t count, const int32
  * (BlockSizeSetup.pas:169-297); this is the persisted form of that step. */
 B2M_API int32_t b2m_batch_tune_save(b2m_ctx* ctx, const char* path);
 B2M_API int32_t b2m_batch_tune_load(b2m_ctx* ctx, const char* path, int32_t* loaded);
-/* The tile shape the autotuner chose for the last batch plan. */
+/* The tile shape the autotuner chose for the last batch plan and its time; a negative time says that the plan was
+ * not tuned (mode 0 has one shape; the other values are then placeholders, in a saved table too). */
 B2M_API int32_t b2m_batch_tune_read(b2m_ctx* ctx, int32_t* small_n, int32_t* group_warps, int32_t* pw_large,
                                     int32_t* pw_small, float* ms);
 

@@ -1518,7 +1518,7 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
         return B2M_OK;
     };
 
-    // mode 0 has one shape: nothing to tune (the table still lists the plan)
+    // mode 0 has one shape: nothing to tune (the table lists the plan, marked by a negative time)
     auto launch_lu = [&](cudaStream_t q) -> int32_t {
         std::atomic<int>& attr = device_flag((const void*)batch_lu_kernel, 0, ctx->device);
         if (!attr.load()) {
@@ -1547,7 +1547,7 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
     if (it != ctx->batch_tunes.end()) {
         best = it->second;
     } else if (mode == 0) {
-        best = ctx->batch_tunes[sig] = BatchTune{64, 1, 32, 16, 8, 0.0f};
+        best = ctx->batch_tunes[sig] = BatchTune{64, 1, 32, 16, 8, -1.0f};
     } else {
         std::vector<BatchTune> cands;
         for (int GB : {8, 4})
@@ -1591,7 +1591,8 @@ int32_t batch_solve(Ctx* ctx, cudaStream_t st, int64_t count, const int32_t* hn,
 // <big_warps> <ms>", after the header line "b2m-batch-tune 2" (a version-1 table, without the
 // big_warps column, is read as big_warps = 8).  A later process that loads the table skips the
 // timing of the candidate shapes for every plan it lists (the signature covers the mode, every
-// system's order, right-hand sides and offsets).
+// system's order, right-hand sides and offsets).  A negative time marks a plan that was not tuned (mode 0): its
+// shape is a placeholder that no kernel uses.
 extern "C" int32_t b2m_batch_tune_save(b2m_ctx* h, const char* path) {
     b2m::Ctx* ctx = reinterpret_cast<b2m::Ctx*>(h);
     if (!ctx || !path) return B2M_ERR_ARG;

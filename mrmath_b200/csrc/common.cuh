@@ -80,7 +80,7 @@ struct BatchTune {
     int pw_large;     // panel widths of the two size buckets
     int pw_small;
     int big_warps;    // warps per system of order > small_n (8: the whole CTA, 4: two per CTA)
-    float ms;         // measured time of the whole batch with this shape
+    float ms;         // measured time of the whole batch with this shape; negative: not tuned (mode 0)
 };
 
 // the batched solve's plan that is on the device (kWsPlan): a host copy of what the caller described it

@@ -298,7 +298,8 @@ def dev_BatchLinEQSolve(n, k, a_off, b_off, A, B, X, info, iters=None, mode: int
 
 
 def batch_tune(ctx=None) -> dict:
-    """The tile shape the batched solve's autotuner chose for the last plan."""
+    """The tile shape the batched solve's autotuner chose for the last plan; a negative `ms` says that it was not
+    tuned (mode 0 has one shape, the fields are placeholders)."""
     vals = [C.c_int32(0) for _ in range(4)]
     ms = C.c_float(0.0)
     c = _ctx_of(ctx)
