@@ -1313,7 +1313,9 @@ int32_t lu_solve_f64(Ctx* ctx, cudaStream_t st, const double* LU, int64_t ld, in
         B2M_CU(ctx, cudaMemcpy2DAsync(X, ldb * 8, B, ldb * 8, nrhs * 8, n, cudaMemcpyDeviceToDevice, s));
         gather_rows_kernel<<<(unsigned)ceil_div(n * nrhs, 256), 256, 0, s>>>(B, ldb, X, ldb, perm, n, nrhs);
         B2M_LAUNCHED(ctx);
-        if (nrhs <= 64) {  // few right-hand sides: block-row sweeps (dtrsv.cu)
+        // few right-hand sides: block-row sweeps (dtrsv.cu), whose workspace and side stream the allocation-free
+        // entry point may not ask for
+        if (nrhs <= 64 && !ctx->fixed_scratch) {
             return tri_solve2_f64(ctx, s, LU, ld, n, kTriL, kTriU, B, ldb, nrhs);
         }
         TriSolve t{LU, ld, n, B, ldb, n, nrhs, 0, nrhs};
