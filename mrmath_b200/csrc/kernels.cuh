@@ -175,9 +175,6 @@ int32_t tf32_split(Ctx* ctx, cudaStream_t st, const float* src, int64_t lds, int
 template <typename T>
 int32_t launch_swaps(Ctx* ctx, cudaStream_t st, T* A, int64_t ld, int ncols, int c0, int w, const int32_t* ipiv,
                      int32_t* perm);
-template <typename T>
-int32_t launch_trsm_small(Ctx* ctx, cudaStream_t st, const T* L, int64_t ldl, T* B, int64_t ldb, int k, int ncols,
-                          bool upper);
 }  // namespace b2m
 
 namespace b2m {

@@ -28,26 +28,6 @@ namespace cg = cooperative_groups;
 
 namespace b2m {
 
-template <typename T> __device__ __forceinline__ T singular_threshold();
-template <> __device__ __forceinline__ double singular_threshold<double>() { return 10.0 / DBL_MAX; }
-template <> __device__ __forceinline__ float singular_threshold<float>() { return 10.0f / FLT_MAX; }
-
-// (a2,i2) beats (a1,i1): larger magnitude, or equal magnitude and lower row (first maximum wins)
-template <typename T>
-__device__ __forceinline__ bool piv_better(T a2, int i2, T a1, int i1) {
-    return i2 >= 0 && (i1 < 0 || a2 > a1 || (a2 == a1 && i2 < i1));
-}
-
-template <typename T>
-__device__ __forceinline__ void warp_argmax(T& a, int& i) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        T a2 = __shfl_xor_sync(0xffffffffu, a, o);
-        int i2 = __shfl_xor_sync(0xffffffffu, i, o);
-        if (piv_better(a2, i2, a, i)) { a = a2; i = i2; }
-    }
-}
-
 constexpr int kPanelW = 32;  // largest leaf width
 
 // ------------------------------------------------------------------------------------------
@@ -1229,16 +1209,7 @@ int32_t launch_swaps(Ctx* ctx, cudaStream_t st, T* A, int64_t ld, int ncols, int
                      int32_t* perm) {
     return launch_swaps_impl<T>(ctx, st, A, ld, ncols, c0, w, ipiv, perm);
 }
-template <typename T>
-int32_t launch_trsm_small(Ctx* ctx, cudaStream_t st, const T* L, int64_t ldl, T* B, int64_t ldb, int k, int ncols,
-                          bool upper) {
-    return launch_trsm_small_impl<T>(ctx, st, L, ldl, B, ldb, k, ncols, upper);
-}
-template int32_t launch_swaps<float>(Ctx*, cudaStream_t, float*, int64_t, int, int, int, const int32_t*, int32_t*);
 template int32_t launch_swaps<double>(Ctx*, cudaStream_t, double*, int64_t, int, int, int, const int32_t*, int32_t*);
-template int32_t launch_trsm_small<float>(Ctx*, cudaStream_t, const float*, int64_t, float*, int64_t, int, int, bool);
-template int32_t launch_trsm_small<double>(Ctx*, cudaStream_t, const double*, int64_t, double*, int64_t, int, int,
-                                           bool);
 
 int32_t lu_factor_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t n, int32_t* ipiv, int32_t* perm) {
     if (n <= 0) return B2M_OK;

@@ -35,12 +35,6 @@ constexpr int kPanelSmemMax = 200 * 1024;  // dynamic shared memory a panel CTA 
 
 template <typename T> __device__ __forceinline__ T sing_thresh();
 template <> __device__ __forceinline__ double sing_thresh<double>() { return 10.0 / DBL_MAX; }
-template <> __device__ __forceinline__ float sing_thresh<float>() { return 10.0f / FLT_MAX; }
-
-template <typename T>
-__device__ __forceinline__ bool better(T a2, int i2, T a1, int i1) {
-    return i2 >= 0 && (i1 < 0 || a2 > a1 || (a2 == a1 && i2 < i1));
-}
 
 // Warp argmax with the reference's tie rule, exactly: |a| >= 0 orders like its bit pattern, so
 // the maximum is found with integer reductions (high word, then low word), and the lowest row
@@ -61,40 +55,13 @@ __device__ __forceinline__ void warp_best(double& a, int& i) {
         i = (int)idx;
     }
 }
-__device__ __forceinline__ void warp_best(float& a, int& i) {
-    const uint32_t key = i >= 0 ? __float_as_uint(a) : 0u;
-    const uint32_t mk = __reduce_max_sync(0xffffffffu, key);
-    const bool top = i >= 0 && key == mk;
-    const uint32_t idx = __reduce_min_sync(0xffffffffu, top ? (uint32_t)i : 0xffffffffu);
-    if (idx == 0xffffffffu) {
-        a = 0.0f;
-        i = -1;
-    } else {
-        a = __uint_as_float(mk);
-        i = (int)idx;
-    }
-}
-
 __device__ __forceinline__ uint4 pack_cand(double a, int i) {
     const unsigned long long b = __double_as_longlong(a);
     return make_uint4((uint32_t)b, (uint32_t)(b >> 32), (uint32_t)i, 0u);
 }
-__device__ __forceinline__ uint4 pack_cand(float a, int i) {
-    return make_uint4(__float_as_uint(a), (uint32_t)i, 0u, 0u);
-}
 __device__ __forceinline__ void unpack_cand(const uint32_t* w, double& a, int& i) {
     a = __longlong_as_double(((unsigned long long)w[1] << 32) | w[0]);
     i = (int)w[2];
-}
-__device__ __forceinline__ void unpack_cand(const uint32_t* w, float& a, int& i) {
-    a = __uint_as_float(w[0]);
-    i = (int)w[1];
-}
-
-__device__ __forceinline__ void st_async_b32(uint32_t raddr, uint32_t v, uint32_t rbar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n" ::"r"(raddr), "r"(v),
-                 "r"(rbar)
-                 : "memory");
 }
 __device__ __forceinline__ void st_async_b64(uint32_t raddr, unsigned long long v, uint32_t rbar) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];\n" ::"r"(raddr), "l"(v),
@@ -104,10 +71,6 @@ __device__ __forceinline__ void st_async_b64(uint32_t raddr, unsigned long long 
 __device__ __forceinline__ void st_async_elem(uint32_t raddr, double v, uint32_t rbar) {
     st_async_b64(raddr, (unsigned long long)__double_as_longlong(v), rbar);
 }
-__device__ __forceinline__ void st_async_elem(uint32_t raddr, float v, uint32_t rbar) {
-    st_async_b32(raddr, __float_as_uint(v), rbar);
-}
-
 // The panel lives in shared memory column-major (S[c*RS + local row], RS odd): a column is a
 // contiguous, conflict-free vector, and a row is one element per lane.
 template <typename T, int W, int RPT>
