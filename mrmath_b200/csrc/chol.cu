@@ -216,8 +216,8 @@ __global__ void copy_lower_kernel(double* dst, int64_t ldd, const double* src, i
 }
 
 // W's upper triangle (diagonal included) <- the transpose of F's lower triangle: 32 x 32 tiles through
-// shared memory, rows read and written whole (3000 x 3000: a
-// copy and an element-wise transpose took 31 + 20 us, this 11)
+// shared memory, rows read and written whole (3000 x 3000: 11 us; a copy and an element-wise transpose
+// took 31 + 20)
 __global__ void __launch_bounds__(256) transpose_lower_kernel(double* W, int64_t ldw, const double* F, int64_t ldf,
                                                               int n) {
     __shared__ double tile[32][33];
@@ -330,8 +330,8 @@ int32_t chol_factor_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_
 }
 
 // Solves A X = B from a Cholesky factor F (lower triangle, diagonal included, row stride ldf):
-// U = L^T is put into the upper triangle of the workspace W (n x ldw), then two FP64 sweeps: L y = b (the transposed upper triangle, true division) and
-// L^T x = y.  B (n x nrhs, ldb) is overwritten with X.
+// U = L^T is put into the upper triangle of the workspace W (n x ldw), then two FP64 sweeps: L y = b (the
+// transposed upper triangle, true division) and L^T x = y.  B (n x nrhs, ldb) is overwritten with X.
 int32_t chol_solve_f64(Ctx* ctx, cudaStream_t st, const double* F, int64_t ldf, int64_t n, double* W, int64_t ldw,
                        double* B, int64_t ldb, int64_t nrhs) {
     if (n <= 0 || nrhs <= 0) return B2M_OK;

@@ -284,9 +284,10 @@ int32_t launch_tile(Ctx* ctx, cudaStream_t st, const DOperand& A, const DOperand
 //   32 x 32, four per SM:         5 + 0.021 K, or 23.5 TFLOP/s over all tiles less 15 %
 //   32 x 16:                      4 + 0.015 K, or 17.5 TFLOP/s less 15 %
 // Measured with 128 x 128 only -> with this choice: 128^3 25.3 -> <= 14.9 us (the call's host time),
-// 1500 x 256 x K 256 (an outer step of the LU) 43.6 -> 15.1, 7900 x 256 x K 256 43.7 (128), 512^3
-// 78.5 -> 19.2, 1024^3 149 -> 84, 1024 x 1 x K 1024 (a residual) 147 -> 18.9, 2999 x 2777 x K 1501
-// 857 -> 795; from 4096^3 on 128 x 128 (3990 us, 64 x 64: 4240).
+// 1500 x 256 x K 256 (an outer step of the LU) 43.1 -> 15.5, 512^3 78.5 -> 19.2, 1024^3 148 -> 84,
+// 1024 x 1 x K 1024 (a residual) 147 -> 18.9, 2999 x 2777 x K 1501 889 -> 835 (subtracting); 128 x 128
+// stays at 1536 x 1536 x K 320 (51 us, 64 x 64: 57) and from 4096^3 on (3986 us, 4250).  Near a line the
+// estimate can miss: 7900 x 256 x K 256 takes 64 x 64 (estimated 43.9 to 44.6), 47.3 us against 43.1.
 int pick_tile(const Ctx* ctx, int64_t M, int64_t N, int64_t K) {
     const double sms = ctx->num_sms, k = (double)K;
     auto tiles = [&](int tm, int tn) { return (double)(ceil_div(M, tm) * ceil_div(N, tn)); };

@@ -724,10 +724,9 @@ __global__ void gather_rows_kernel(double* X, int64_t ldx, const double* B, int6
 //     V(j) = V(k), k the last k < j with ipiv[k] = j, or j if there is none;
 //     perm[i] = V(i) if ipiv[i] = i, else V(k), k the last k < i with ipiv[k] = ipiv[i], or ipiv[i].
 // The first k is a maximum over all interchanges; the second comes from one warp walking the steps 32
-// at a time with a table of the last interchange per position; V by pointer jumping.  One thread's
-// sequential interchanges (140 cycles each) remain for other vectors and orders: order 4096 took
-// 283 us, now
-// 37.
+// at a time with a table of the last interchange per position; V by pointer jumping.  Order 4096 takes
+// 37 us; one thread's sequential interchanges (140 cycles each), which remain for other vectors and
+// orders, take 283.
 constexpr int kPermThreads = 1024;
 constexpr uint16_t kPermNone = 0xffff;
 constexpr int kPermMax = 32768;  // orders whose three tables of 16-bit indices fit shared memory
@@ -1012,8 +1011,10 @@ static_assert(kOuterNB == kTpK, "the panel triangular solve holds one outer pane
 
 // Blocked right-looking LU with look-ahead (orders n > kSmallLu).  Per outer panel of 256
 // columns: (1) the panel is factored right-looking by leaves, each leaf's interchanges kept inside
-// the panel (and recorded in the row map pmap), its U12 formed by the same launch and its rank-w
-// update applied to the rest of the panel (leaf_swap_u12_kernel, panel_rank_update_kernel); (2) the
+// the panel (and recorded in the row map pmap), its U12 and its rank-w update applied to the rest of
+// the panel (to the next leaf by that leaf's own kernel, beyond it by leaf_side_kernel and
+// panel_rank_update_kernel; leaves of 16 or 8 columns by leaf_swap_u12_kernel and
+// panel_rank_update_kernel); (2) the
 // panel's net permutation is applied to the next panel's columns on this stream, and to every
 // further column right of the panel and the factored columns left of it on the side stream;
 // (3) U12 = L11^-1 A12 (trsm_panel_kernel, one launch) and A22 -= A21 U12 for the next panel's
@@ -1057,8 +1058,8 @@ int32_t lu_blocked(Ctx* ctx, cudaStream_t q, double* A, int64_t ld, int64_t n, i
         }
         // The panel, right-looking by leaves.  The critical path, on this stream: a leaf's panel
         // kernel, then its interchanges, U12 and rank-w update on the next leaf's columns only (in the
-        // next leaf's own kernel when the leaves are linked); the same for the other columns of the outer panel (the factored ones left of the leaf get the
-        // interchanges only) runs on the leaf stream, under the next leaf's panel kernel, and is
+        // next leaf's own kernel when the leaves are linked); the same for the other columns of the
+        // outer panel (the factored ones left of the leaf get the interchanges only) runs on the leaf stream, under the next leaf's panel kernel, and is
         // waited for before that leaf's own updates touch those columns.  Column groups are
         // disjoint between the two streams, and every column sees the leaves' interchanges and
         // updates in leaf order, so the factors are those of the single-stream order.

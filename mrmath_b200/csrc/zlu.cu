@@ -30,8 +30,8 @@ namespace {
 
 constexpr int kZLeaf = 32;
 constexpr int kZPanelThreads = 1024;
-// Widest block without GEMMs.  The line hardly matters: order 2048 took 11.9, 11.3 and 11.3 ms with 256, 1024
-// and 4096 (two right-hand sides), the inverse-like solve with 2048 right-hand sides 35.4 to 36.3 ms.
+// Widest block without GEMMs.  For the factorisation the line hardly matters (order 2048 took 11.9, 11.3 and 11.3
+// ms with 256, 1024 and 4096); solves with many right-hand sides want the GEMMs above it (see zlu_solve).
 constexpr int64_t kZBlock = 1024;
 
 struct Planes {
@@ -976,8 +976,12 @@ int32_t zlu_solve(Ctx* ctx, cudaStream_t st, const double* lre, const double* li
     if (n <= 0 || nrhs <= 0) return B2M_OK;
     const Planes L{const_cast<double*>(lre), const_cast<double*>(lim), ld};
     const Planes X{bre, bim, ldb}, W{tre, tim, ldb};
-    // steps of 32 rows out of place (so that several CTAs can share a strip's rows) while the right-hand sides
-    // are few or the steps are short; else in place, split into GEMMs above kZBlock
+    // Steps of 32 rows out of place (so that several CTAs can share a strip's rows) while the right-hand sides
+    // are few or the matrix is one block; else in place, split into GEMMs above kZBlock.  Kernels of a solve, steps
+    // against GEMMs, ms: order 1100 64 right-hand sides 0.93 / 1.35, 256 1.03 / 1.39, 2048 2.06 / 1.88; order 2048
+    // 1.85 / 3.48, 2.21 / 3.61, 5.66 / 4.83; order 3000 2.8 / 5.0, 3.6 / 5.2, 12.1 / 9.2.  The two meet between
+    // 1000 and 2000 right-hand sides; from the line up to there the GEMMs cost up to 45 % more (order 2048, 512:
+    // 2.7 / 3.9), and the line has not been moved.
     const bool steps = nrhs <= 256 || n <= kZBlock;
     const Planes& G = steps ? W : X;
     if (!steps) {
