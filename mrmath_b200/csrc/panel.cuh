@@ -28,6 +28,12 @@ static __device__ __noinline__ int warp_winner(double a, int pos) {
 // of it and leaves the elimination together: which barriers a thread meets never depends on what it saw alone.
 // A warp that has not given up has seen every candidate so far, so what it records is always a valid interchange.
 
+// (out of line: inlined into panel_kernel's column loop it cost 1 to 2 % of a leaf)
+static __device__ __noinline__ void cluster_give_up(int* late, int C, int32_t* status, int site) {
+    atomicExch(&status[kTimeout], site);
+    for (int d = 0; d < C; ++d)
+        asm volatile("st.shared::cluster.u32 [%0], 1;\n" ::"r"(map_rank(late, d)) : "memory");
+}
 // waits for a phase of this CTA's barrier, for `polls` polls or until a thread of the cluster has given up; false: in vain
 __device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t phase, uint32_t polls, int* late, int C,
                                              int32_t* status, int site) {
@@ -35,9 +41,7 @@ __device__ __forceinline__ bool cluster_wait(uint64_t* bar, uint32_t phase, uint
         if (mbar_try_wait_cluster(bar, phase)) return true;
         if ((it & 255u) == 255u && *reinterpret_cast<volatile int*>(late) != 0) break;
     }
-    atomicExch(&status[kTimeout], site);
-    for (int d = 0; d < C; ++d)
-        asm volatile("st.shared::cluster.u32 [%0], 1;\n" ::"r"(map_rank(late, d)) : "memory");
+    cluster_give_up(late, C, status, site);
     return false;
 }
 // A cluster kernel's end: no CTA leaves while a push to it may be in flight.  Every push that was waited for has
