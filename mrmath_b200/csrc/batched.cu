@@ -1207,8 +1207,8 @@ __global__ void __launch_bounds__(kLuThreads, kLuCtas) batch_lu_kernel(BatchArgs
 //
 // small_lu_kernel: four warps do the leaves, eight the strips.  L is kept too, in its storage row; rows go to
 // their positions at the end, from the scratch V (n rows of (n + 1) & ~1) back to A.
-// Measured on a B200 (factor and one right-hand side, the whole call): order 100 201 us before and 126 us now,
-// order 256 429 and 350 us; the inverse of order 100 230 and 129 us.
+// Measured on a B200 (factor and one right-hand side, the whole call): order 100 201 us before and 125 us now,
+// order 256 429 and 339 us; the inverse of order 100 230 and 129 us.
 // ------------------------------------------------------------------------------------------
 constexpr int kSmThreads = 256;
 

@@ -1228,9 +1228,9 @@ int32_t lu_factor_f64(Ctx* ctx, cudaStream_t st, double* A, int64_t ld, int64_t 
         ctx->progress_notes.reserve((size_t)(n / 8 + 2));
     }
     // Three ways, by the order (measured, factor + solve of one right-hand side, us):
-    //   * up to 256 (kSmallLu), one launch of one CTA (order 16: 36 against 44 by the recursion, 100: 126 / 201,
-    //     256: 350 / 429 and about 375 by the blocked driver);
-    //   * above, the blocked look-ahead driver with linked leaves (257: 377 / 491, 512: 658 / 931);
+    //   * up to 256 (kSmallLu), one launch of one CTA (order 16: 33 against 44 by the recursion, 100: 125 / 201,
+    //     256: 339 / 429 and about 375 by the blocked driver);
+    //   * above, the blocked look-ahead driver with linked leaves (257: 366 / 491, 512: 652 / 931);
     //   * the plain recursion where no workspace or side stream may be used (the allocation-free entry
     //     point, n <= 512).
     // Every order asks for the small orders' scratch and the side streams, so that after a call of any order
